@@ -65,6 +65,11 @@ int32_t pb_accumulate_rho(const float* x, const float* y, float* rho, int32_t nu
 int32_t pb_accumulate_rho_noalloc(const float* x, const float* y, float* rho, int32_t num_p, double dx, double dy,
                                   int32_t nx, int32_t ny, double charge_density, void* stream);
 
+/* pb_push_particles_boris (large calls), pb_accumulate_rho and pb_compute_particle_substeps
+ * take their scratch from a stream-ordered memory pool of the library's own, which keeps up to
+ * 256 MB per context between calls.  This gives what is not in use back to the device. */
+int32_t pb_release_scratch(void);
+
 /* Exhaustive check of the division the step kernels use for x / dx and y / dy (no
  * counterpart in the reference; a test of this library).  For the float32 spacing d, every
  * one of the 2^32 float32 values x is divided by bracketing (x * RN(1/d), its FMA residual

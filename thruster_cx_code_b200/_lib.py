@@ -74,6 +74,7 @@ PROTOTYPES = {
     "pb_thermal_conduction": (i32, [vp, vp, vp, i32, i32, f64, f64, vp]),
     "pb_compute_particle_substeps": (i32, [vp, vp, vp, vp, vp, i32, vp, vp, i32, i32, f64, f64, f64, f64, f64, P(f64), vp]),
     "pb_segment_hits_grid": (i32, [vp, i32, i32, f64, f64, vp, vp, vp, vp, i32, vp, vp, vp, vp]),
+    "pb_release_scratch": (i32, []),
     "pb_sim_create": (i32, [P(vp), i32]),
     "pb_sim_destroy": (i32, [vp]),
     "pb_sim_set_seed": (i32, [vp, u64]),

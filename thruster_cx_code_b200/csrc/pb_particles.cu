@@ -35,6 +35,15 @@ __device__ __forceinline__ double gather4(const float* __restrict__ F, size_t r0
   return DADD(DADD(DADD(a, b), c), d);
 }
 
+// The two float4 of one cell's corners (32 bytes, 32-byte aligned) in one load.  A gather of
+// particles in scattered cells is bound by the cache's tag lookups, one per lane and load
+// instruction, so one 256-bit load instead of two of 128 bits halves them.
+__device__ __forceinline__ void ldg_corners(const float4* __restrict__ p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
 // The same from the per-cell corner array: Ec[2c] holds Ex at (iy0, ix0), (iy0, ix0 + 1),
 // (iy0 + 1, ix0), (iy0 + 1, ix0 + 1) of cell c = iy0 * nx + ix0, Ec[2c + 1] the same of
 // Ey: one 16-byte load per component instead of four scalar loads, same arithmetic.
@@ -47,7 +56,9 @@ __device__ __forceinline__ void gather4v(const float4 a, const float4 b, double 
 }
 __device__ __forceinline__ void gather4c(const float4* __restrict__ Ec, size_t c, double w00, double w10,
                                          double w01, double w11, double& ex, double& ey) {
-  gather4v(__ldg(Ec + 2 * c), __ldg(Ec + 2 * c + 1), w00, w10, w01, w11, ex, ey);
+  float4 a, b;
+  ldg_corners(Ec + 2 * c, a, b);
+  gather4v(a, b, w00, w10, w01, w11, ex, ey);
 }
 
 // The window of the corner array staged in shared memory for a tile (PB_OPT_TMA_TILE):
@@ -278,6 +289,29 @@ __device__ __forceinline__ void push_update_b0(float& x, float& y, float& vx, fl
   y = __fadd_rn(y, __fmul_rn(__fmul_rn(vy, dtf), 1000.0f));
 }
 
+// Half kick, rotation, half kick and drift from the gathered E and B.
+__device__ __forceinline__ void push_update_b(float& x, float& y, float& vx, float& vy, float& vz, double ex, double ey,
+                                              double bx, double by, double bz, double h, float dtf) {
+  const double vmx = DADD((double)vx, DMUL(h, ex));
+  const double vmy = DADD((double)vy, DMUL(h, ey));
+  const double vmz = (double)vz;
+  const double tx = DMUL(h, bx), ty = DMUL(h, by), tz = DMUL(h, bz);
+  const double t2 = DADD(DADD(DMUL(tx, tx), DMUL(ty, ty)), DMUL(tz, tz));
+  const double den = DADD(1.0, t2);
+  const double sx = DDIV(DMUL(2.0, tx), den), sy = DDIV(DMUL(2.0, ty), den), sz = DDIV(DMUL(2.0, tz), den);
+  const double vpx = DADD(vmx, DSUB(DMUL(vmy, tz), DMUL(vmz, ty)));
+  const double vpy = DADD(vmy, DSUB(DMUL(vmz, tx), DMUL(vmx, tz)));
+  const double vpz = DADD(vmz, DSUB(DMUL(vmx, ty), DMUL(vmy, tx)));
+  const double wx = DADD(vmx, DSUB(DMUL(vpy, sz), DMUL(vpz, sy)));
+  const double wy = DADD(vmy, DSUB(DMUL(vpz, sx), DMUL(vpx, sz)));
+  const double wz = DADD(vmz, DSUB(DMUL(vpx, sy), DMUL(vpy, sx)));
+  vx = __double2float_rn(DADD(wx, DMUL(h, ex)));
+  vy = __double2float_rn(DADD(wy, DMUL(h, ey)));
+  vz = __double2float_rn(wz);
+  x = __fadd_rn(x, __fmul_rn(__fmul_rn(vx, dtf), 1000.0f));
+  y = __fadd_rn(y, __fmul_rn(__fmul_rn(vy, dtf), 1000.0f));
+}
+
 template <bool HAS_B, bool CORN = false, bool LIGHT = false>
 __device__ __forceinline__ void boris_push_one(float& x, float& y, float& vx, float& vy, float& vz,
                                                const float* __restrict__ Ex, const float* __restrict__ Ey,
@@ -302,8 +336,9 @@ __device__ __forceinline__ void boris_push_one(float& x, float& y, float& vx, fl
       gather4v(q[0], q[1], w00, w10, w01, w11, ex, ey);
     } else {
       if (LIGHT) {  // 32-bit cell index (a grid has fewer than 2^30 cells): fewer instructions
-        const float4* e = Ec + 2 * (iy0 * nx + ix0);
-        gather4v(__ldg(e), __ldg(e + 1), w00, w10, w01, w11, ex, ey);
+        float4 ea, eb4;
+        ldg_corners(Ec + 2 * (iy0 * nx + ix0), ea, eb4);
+        gather4v(ea, eb4, w00, w10, w01, w11, ex, ey);
       } else {
         gather4c(Ec, r0 + ix0, w00, w10, w01, w11, ex, ey);
       }
@@ -316,27 +351,10 @@ __device__ __forceinline__ void boris_push_one(float& x, float& y, float& vx, fl
     push_update_b0(x, y, vx, vy, vz, ex, ey, h, dtf);
     return;
   }
-  const double vmx = DADD((double)vx, DMUL(h, ex));
-  const double vmy = DADD((double)vy, DMUL(h, ey));
-  const double vmz = (double)vz;
-  double bx = gather4(Bx, r0, r1, ix0, ix1, w00, w10, w01, w11);
-  double by = gather4(By, r0, r1, ix0, ix1, w00, w10, w01, w11);
-  double bz = gather4(Bz, r0, r1, ix0, ix1, w00, w10, w01, w11);
-  const double tx = DMUL(h, bx), ty = DMUL(h, by), tz = DMUL(h, bz);
-  const double t2 = DADD(DADD(DMUL(tx, tx), DMUL(ty, ty)), DMUL(tz, tz));
-  const double den = DADD(1.0, t2);
-  const double sx = DDIV(DMUL(2.0, tx), den), sy = DDIV(DMUL(2.0, ty), den), sz = DDIV(DMUL(2.0, tz), den);
-  const double vpx = DADD(vmx, DSUB(DMUL(vmy, tz), DMUL(vmz, ty)));
-  const double vpy = DADD(vmy, DSUB(DMUL(vmz, tx), DMUL(vmx, tz)));
-  const double vpz = DADD(vmz, DSUB(DMUL(vmx, ty), DMUL(vmy, tx)));
-  const double wx = DADD(vmx, DSUB(DMUL(vpy, sz), DMUL(vpz, sy)));
-  const double wy = DADD(vmy, DSUB(DMUL(vpz, sx), DMUL(vpx, sz)));
-  const double wz = DADD(vmz, DSUB(DMUL(vpx, sy), DMUL(vpy, sx)));
-  vx = __double2float_rn(DADD(wx, DMUL(h, ex)));
-  vy = __double2float_rn(DADD(wy, DMUL(h, ey)));
-  vz = __double2float_rn(wz);
-  x = __fadd_rn(x, __fmul_rn(__fmul_rn(vx, dtf), 1000.0f));
-  y = __fadd_rn(y, __fmul_rn(__fmul_rn(vy, dtf), 1000.0f));
+  const double bx = gather4(Bx, r0, r1, ix0, ix1, w00, w10, w01, w11);
+  const double by = gather4(By, r0, r1, ix0, ix1, w00, w10, w01, w11);
+  const double bz = gather4(Bz, r0, r1, ix0, ix1, w00, w10, w01, w11);
+  push_update_b(x, y, vx, vy, vz, ex, ey, bx, by, bz, h, dtf);
 }
 
 // Two electrons pushed n_sub times side by side (PB_OPT_ELE_PAIRS): both cells and both
@@ -354,8 +372,7 @@ __device__ __forceinline__ void push_pair_b0(float (&x)[2], float (&y)[2], float
       push_cell<true>(x[q], y[q], nx, ny, dxf, dyf, rc, nullptr, ix0[q], iy0[q], w[q][0], w[q][1],
                       w[q][2], w[q][3]);
       const size_t c = (size_t)iy0[q] * nx + ix0[q];
-      A[q] = __ldg(Ec + 2 * c);
-      B[q] = __ldg(Ec + 2 * c + 1);
+      ldg_corners(Ec + 2 * c, A[q], B[q]);
     }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -384,6 +401,126 @@ __global__ void k_push_boris(float* x, float* y, float* vx, float* vy, float* vz
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float a = x[i], b = y[i], c = vx[i], d = vy[i], e = vz[i];
     boris_push_one<true>(a, b, c, d, e, Ex, Ey, Bx, By, Bz, nx, ny, dxf, dyf, h, dtf);
+    x[i] = a; y[i] = b; vx[i] = c; vy[i] = d; vz[i] = e;
+  }
+}
+
+// ------------------------------------------------------------------ standalone push, many particles
+// With many particles per cell the push above is bound by the sectors of its 20 scalar
+// gathers (ten 32-byte sectors a particle: L1 94% and L2 72% busy, DRAM 8%, 878 us for 16M
+// ions on 513 x 2049).  Packing the corners of every cell first (as the step does) makes E one
+// sector a particle and B two, for one pass over the grid.  k_push_corners packs E and leaves
+// per block whether any B bit is set; with every B value +0 (the reference's step) the B = 0
+// push is the same operation (boris_push_one) and no B is gathered, otherwise k_push_bcorners
+// packs B too.  Both pushes are launched and the wrong one returns at once, so the host need
+// not wait for the flag.  16M ions on 513 x 2049: 878 us before, 170 us packed (143 us of it
+// the push, 640 MB of particle state: 4.5 TB/s); with a B field 880 and 435 us.
+constexpr int PUSH_FLAGS = 1184;  // blocks of k_push_corners, one flag each
+
+__global__ void __launch_bounds__(256) k_push_corners(const float* __restrict__ Ex, const float* __restrict__ Ey,
+                                                      const float* __restrict__ Bx, const float* __restrict__ By,
+                                                      const float* __restrict__ Bz, float4* __restrict__ Ec, int ny,
+                                                      int nx, unsigned* __restrict__ bflags) {
+  const int N = ny * nx;
+  unsigned bits = 0u;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+    bits |= __float_as_uint(__ldg(Bx + c)) | __float_as_uint(__ldg(By + c)) | __float_as_uint(__ldg(Bz + c));
+    const int iy = c / nx, ix = c - iy * nx;
+    if (iy >= ny - 1 || ix >= nx - 1) continue;
+    const int r1 = c + nx;
+    Ec[2 * c] = make_float4(__ldg(Ex + c), __ldg(Ex + c + 1), __ldg(Ex + r1), __ldg(Ex + r1 + 1));
+    Ec[2 * c + 1] = make_float4(__ldg(Ey + c), __ldg(Ey + c + 1), __ldg(Ey + r1), __ldg(Ey + r1 + 1));
+  }
+  const int any = __syncthreads_or(bits != 0u);
+  if (threadIdx.x == 0) bflags[blockIdx.x] = any ? 1u : 0u;
+}
+
+// whether any block of k_push_corners saw a B bit (every thread of the block calls it)
+__device__ __forceinline__ bool push_any_b(const unsigned* __restrict__ bflags, int nflags) {
+  unsigned f = 0u;
+  for (int k = threadIdx.x; k < nflags; k += blockDim.x) f |= __ldg(bflags + k);
+  return __syncthreads_or(f != 0u) != 0;
+}
+
+// B corners of cell c: Bc[2 c], Bc[2 c + 1] are Bx, By at (iy0, ix0), (iy0, ix0 + 1), (iy0 + 1, ix0),
+// (iy0 + 1, ix0 + 1), Bc[2 N + c] the same of Bz
+__global__ void __launch_bounds__(256) k_push_bcorners(const float* __restrict__ Bx, const float* __restrict__ By,
+                                                       const float* __restrict__ Bz, float4* __restrict__ Bc, int ny,
+                                                       int nx, const unsigned* __restrict__ bflags, int nflags) {
+  pdl_enter();
+  if (!push_any_b(bflags, nflags)) return;
+  const int N = ny * nx;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+    const int iy = c / nx, ix = c - iy * nx;
+    if (iy >= ny - 1 || ix >= nx - 1) continue;
+    const int r1 = c + nx;
+    Bc[2 * c] = make_float4(__ldg(Bx + c), __ldg(Bx + c + 1), __ldg(Bx + r1), __ldg(Bx + r1 + 1));
+    Bc[2 * c + 1] = make_float4(__ldg(By + c), __ldg(By + c + 1), __ldg(By + r1), __ldg(By + r1 + 1));
+    Bc[2 * N + c] = make_float4(__ldg(Bz + c), __ldg(Bz + c + 1), __ldg(Bz + r1), __ldg(Bz + r1 + 1));
+  }
+}
+
+template <bool HAS_B>
+__device__ __forceinline__ void push_corner_one(float& x, float& y, float& vx, float& vy, float& vz,
+                                                const float4* __restrict__ Ec, const float4* __restrict__ Bc, int nx,
+                                                int ny, float dxf, float dyf, double h, float dtf, const Rcp& rc) {
+  if (!HAS_B) {
+    boris_push_one<false, true, true>(x, y, vx, vy, vz, nullptr, nullptr, nullptr, nullptr, nullptr, nx, ny, dxf, dyf, h,
+                                      dtf, Ec, rc);
+    return;
+  }
+  int ix0, iy0;
+  double w00, w10, w01, w11;
+  push_cell<true>(x, y, nx, ny, dxf, dyf, rc, nullptr, ix0, iy0, w00, w10, w01, w11);
+  const int c = iy0 * nx + ix0;
+  float4 ea, eb, ba, bb;
+  ldg_corners(Ec + 2 * c, ea, eb);
+  ldg_corners(Bc + 2 * c, ba, bb);
+  const float4 bc = __ldg(Bc + 2 * nx * ny + c);
+  double ex, ey, bx, by, bz, unused;
+  gather4v(ea, eb, w00, w10, w01, w11, ex, ey);
+  gather4v(ba, bb, w00, w10, w01, w11, bx, by);
+  gather4v(bc, bc, w00, w10, w01, w11, bz, unused);
+  push_update_b(x, y, vx, vy, vz, ex, ey, bx, by, bz, h, dtf);
+}
+
+// VEC: the five arrays start 16-byte aligned (four particles per thread and pass, 16-byte
+// loads and stores); the last n % 4 particles, and all of them otherwise, go one by one.
+// Four blocks an SM (64 registers): 152 us for the 16M ions, against 193 us at 78 registers,
+// 169 us at 40 and 176 us one particle a thread at 32; a software prefetch of the next four
+// particles (78 registers) 192 us.
+template <bool HAS_B, bool VEC>
+__global__ void __launch_bounds__(256, 4) k_push_corner(float* __restrict__ x, float* __restrict__ y,
+                                                     float* __restrict__ vx, float* __restrict__ vy,
+                                                     float* __restrict__ vz, const float4* __restrict__ Ec,
+                                                     const float4* __restrict__ Bc, int n, int nx, int ny, float dxf,
+                                                     float dyf, double h, float dtf, Rcp rc,
+                                                     const unsigned* __restrict__ bflags, int nflags) {
+  pdl_enter();
+  if (push_any_b(bflags, nflags) != HAS_B) return;
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  int done = 0;
+  if (VEC) {
+    const int n4 = n >> 2;
+    done = n4 << 2;
+    for (int q = t0; q < n4; q += stride) {
+      float4 X = reinterpret_cast<float4*>(x)[q], Y = reinterpret_cast<float4*>(y)[q];
+      float4 U = reinterpret_cast<float4*>(vx)[q], V = reinterpret_cast<float4*>(vy)[q];
+      float4 W = reinterpret_cast<float4*>(vz)[q];
+      push_corner_one<HAS_B>(X.x, Y.x, U.x, V.x, W.x, Ec, Bc, nx, ny, dxf, dyf, h, dtf, rc);
+      push_corner_one<HAS_B>(X.y, Y.y, U.y, V.y, W.y, Ec, Bc, nx, ny, dxf, dyf, h, dtf, rc);
+      push_corner_one<HAS_B>(X.z, Y.z, U.z, V.z, W.z, Ec, Bc, nx, ny, dxf, dyf, h, dtf, rc);
+      push_corner_one<HAS_B>(X.w, Y.w, U.w, V.w, W.w, Ec, Bc, nx, ny, dxf, dyf, h, dtf, rc);
+      reinterpret_cast<float4*>(x)[q] = X;
+      reinterpret_cast<float4*>(y)[q] = Y;
+      reinterpret_cast<float4*>(vx)[q] = U;
+      reinterpret_cast<float4*>(vy)[q] = V;
+      reinterpret_cast<float4*>(vz)[q] = W;
+    }
+  }
+  for (int i = done + t0; i < n; i += stride) {
+    float a = x[i], b = y[i], c = vx[i], d = vy[i], e = vz[i];
+    push_corner_one<HAS_B>(a, b, c, d, e, Ec, Bc, nx, ny, dxf, dyf, h, dtf, rc);
     x[i] = a; y[i] = b; vx[i] = c; vy[i] = d; vz[i] = e;
   }
 }
@@ -527,7 +664,8 @@ __device__ __forceinline__ double predicted_ds(float x, float y, float vx, float
   size_t r0 = (size_t)iy0 * nx, r1 = (size_t)(iy0 + 1) * nx;
   double ex, ey;
   if (Ec) {
-    const float4 a = __ldg(Ec + 2 * (r0 + ix0)), b = __ldg(Ec + 2 * (r0 + ix0) + 1);
+    float4 a, b;
+    ldg_corners(Ec + 2 * (r0 + ix0), a, b);
     const double gx = DSUB(1.0, fx), gy = DSUB(1.0, fy);
     ex = DADD(DADD(DADD(DMUL(DMUL((double)a.x, gx), gy), DMUL(DMUL((double)a.y, fx), gy)),
                    DMUL(DMUL((double)a.z, gx), fy)), DMUL(DMUL((double)a.w, fx), fy));
@@ -1283,8 +1421,8 @@ __device__ __forceinline__ void ele_substep(float& x, float& y, float& vx, float
   const double gx = DSUB(1.0, fx), gy = DSUB(1.0, fy);
   const double w00 = DMUL(gx, gy), w10 = DMUL(fx, gy), w01 = DMUL(gx, fy), w11 = DMUL(fx, fy);
   const double w00s = DMUL(w00, 0x1p896);
-  const float4* e = a.Ec + 2 * (fyi * a.nx + fxi);
-  const float4 A = __ldg(e), B = __ldg(e + 1);
+  float4 A, B;
+  ldg_corners(a.Ec + 2 * (fyi * a.nx + fxi), A, B);
   const double ex = DADD(DADD(DADD(DMUL(f2d_scaled(A.x), w00s), DMUL((double)A.y, w10)), DMUL((double)A.z, w01)),
                          DMUL((double)A.w, w11));
   const double ey = DADD(DADD(DADD(DMUL(f2d_scaled(B.x), w00s), DMUL((double)B.y, w10)), DMUL((double)B.z, w01)),

@@ -38,11 +38,108 @@ static int32_t fail(int32_t code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail(PB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// ------------------------------------------------------------------ scratch of the module-level entry points
+// A stream-ordered memory pool of the library's own, one per context, that keeps up to
+// SCRATCH_KEEP bytes across synchronisations.  The device's default pool gives its memory back
+// whenever the stream is synchronised, so a call that allocated from it took 480 us to several
+// ms when the caller waited for each result (deposit of 100k particles: 34 us back to back).
+// Allocation and release are ordered on the caller's stream, so calls on several streams and
+// threads never share memory that is in use.  A capturing stream, and anything unexpected,
+// takes the default pool as before.  pb_release_scratch gives unused memory back, and so does
+// an allocation of the simulator's own that finds the device full.
+constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
+struct ScratchPool {
+  unsigned long long ctx = 0;
+  cudaMemPool_t pool = nullptr;
+};
+static std::mutex g_scratch_mu;
+static ScratchPool g_scratch[16];  // contexts beyond these use the default pool
+
+// the id of the context current on this thread (never reused, unlike its address); 0 if unknown
+static unsigned long long current_context_id() {
+  typedef CUresult (*GetCurrentFn)(CUcontext*);
+  typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
+  static GetCurrentFn get_current = nullptr;
+  static GetIdFn get_id = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_current = reinterpret_cast<GetCurrentFn>(p);
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_id = reinterpret_cast<GetIdFn>(p);
+  });
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (!get_current || !get_id || get_current(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0;
+  return id;
+}
+
+// the pool of the current context, or nullptr
+static cudaMemPool_t scratch_pool(bool create) {
+  unsigned long long id = current_context_id();
+  if (!id) {
+    if (!create || cudaFree(nullptr) != cudaSuccess || !(id = current_context_id())) return nullptr;
+  }
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  for (ScratchPool& s : g_scratch) {
+    if (s.ctx == id) return s.pool;
+    if (s.ctx || !create) continue;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    uint64_t keep = SCRATCH_KEEP;
+    s.ctx = id;  // a context whose pool cannot be made keeps nullptr: the default pool
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another thread may be capturing
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemPoolCreate(&s.pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+      s.pool = nullptr;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return s.pool;
+  }
+  return nullptr;
+}
+
+static bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(st, &cs);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+static cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+  *p = nullptr;
+  if (!stream_capturing(st)) {
+    if (cudaMemPool_t pool = scratch_pool(true)) {
+      if (cudaMallocFromPoolAsync(p, bytes, pool, st) == cudaSuccess) return cudaSuccess;
+      cudaGetLastError();
+      *p = nullptr;
+    }
+  }
+  return cudaMallocAsync(p, bytes, st);
+}
+
+static void scratch_trim() {
+  if (cudaMemPool_t pool = scratch_pool(false)) cudaMemPoolTrimTo(pool, 0);
+}
+
 template <typename T>
 static cudaError_t dalloc(T** p, size_t n) {
   *p = nullptr;
   if (n == 0) n = 1;
-  return cudaMalloc((void**)p, n * sizeof(T));
+  cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    scratch_trim();
+    e = cudaMalloc((void**)p, n * sizeof(T));
+  }
+  return e;
 }
 template <typename T>
 static void dfree(T*& p) {
@@ -1912,6 +2009,15 @@ int32_t pb_check_division(double d, int64_t* out3) {
   return PB_OK;
 }
 
+int32_t pb_release_scratch(void) {
+  scratch_trim();
+  return PB_OK;
+}
+
+// Where pb_push_particles_boris packs the corners first
+constexpr int PUSH_PACK_MIN = 600000;
+constexpr long long PUSH_PACK_CELLS = 4ll << 20;  // at most 320 MB of corners
+
 int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float* vz, const float* Ex, const float* Ey,
                                 const float* Bx, const float* By, const float* Bz, int32_t num_p, double dx, double dy,
                                 int32_t nx, int32_t ny, double dt, double q_m, void* stream) {
@@ -1919,9 +2025,47 @@ int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float*
   if (nx < 2 || ny < 2) return fail(PB_ERR_ARG, "push: grid must be at least 2 x 2");
   double h = (0.5 * q_m) * dt;
   int bs = 256;
+  cudaStream_t st = (cudaStream_t)stream;
+  const long long cells = (long long)nx * ny;
+  // Corners packed first (k_push_corners) where the gathers saved pay for the pass over the
+  // grid and three more launches.  Measured, direct against packed (us): 65 x 284 nodes 20
+  // against 26 at 400k particles, 41 against 26 at 1M; 257 x 1025 27 against 19 (27 with a B
+  // field) at 400k, 59 against 23 (39) at 1M; 513 x 2049 60 against 33 (72) at 1M, 225 against
+  // 61 (132) at 4M.  So from 600k particles and 1.5 a cell.  A capturing stream keeps the one
+  // launch, which needs no memory.
+  if (num_p >= PUSH_PACK_MIN && (long long)num_p * 2 >= 3 * cells && cells <= PUSH_PACK_CELLS && !stream_capturing(st)) {
+    const size_t fl = ((PUSH_FLAGS * sizeof(unsigned) + 255) / 256) * 256;
+    char* ws = nullptr;
+    if (scratch_alloc((void**)&ws, fl + (size_t)cells * 5 * sizeof(float4), st) == cudaSuccess) {
+      unsigned* flags = reinterpret_cast<unsigned*>(ws);
+      float4* ec = reinterpret_cast<float4*>(ws + fl);
+      float4* bc = ec + 2 * cells;
+      const float dxf = (float)dx, dyf = (float)dy, dtf = (float)dt;
+      const Rcp rc = make_rcp(dxf, dyf);
+      const int gc = (int)std::min<long long>((cells + bs - 1) / bs, PUSH_FLAGS);
+      const bool vec = (((uintptr_t)x | (uintptr_t)y | (uintptr_t)vx | (uintptr_t)vy | (uintptr_t)vz) & 15u) == 0;
+      const long per = vec ? 4 : 1;
+      const int gp = (int)std::min<long>((num_p / per + bs) / bs, 148L * 4);
+      k_push_corners<<<gc, bs, 0, st>>>(Ex, Ey, Bx, By, Bz, ec, ny, nx, flags);
+      cudaError_t e = cudaGetLastError();
+      const unsigned* cf = flags;
+      const float4 *cec = ec, *cbc = bc;
+      if (e == cudaSuccess) e = launch_pdl(k_push_bcorners, gc, bs, 0, st, Bx, By, Bz, bc, ny, nx, cf, gc);
+      if (e == cudaSuccess)
+        e = launch_pdl(vec ? k_push_corner<true, true> : k_push_corner<true, false>, gp, bs, 0, st, x, y, vx, vy, vz,
+                       cec, cbc, num_p, nx, ny, dxf, dyf, h, dtf, rc, cf, gc);
+      if (e == cudaSuccess)
+        e = launch_pdl(vec ? k_push_corner<false, true> : k_push_corner<false, false>, gp, bs, 0, st, x, y, vx, vy, vz,
+                       cec, cbc, num_p, nx, ny, dxf, dyf, h, dtf, rc, cf, gc);
+      const cudaError_t ef = cudaFreeAsync(ws, st);
+      CK(e);
+      CK(ef);
+      return PB_OK;
+    }
+    cudaGetLastError();  // no memory for the corners: the push without them
+  }
   int g = (int)std::min<long>((num_p + bs - 1) / bs, 148L * 16);
-  k_push_boris<<<g, bs, 0, (cudaStream_t)stream>>>(x, y, vx, vy, vz, Ex, Ey, Bx, By, Bz, num_p, nx, ny, (float)dx,
-                                                   (float)dy, h, (float)dt);
+  k_push_boris<<<g, bs, 0, st>>>(x, y, vx, vy, vz, Ex, Ey, Bx, By, Bz, num_p, nx, ny, (float)dx, (float)dy, h, (float)dt);
   CK(cudaGetLastError());
   return PB_OK;
 }
@@ -1936,7 +2080,7 @@ int32_t pb_accumulate_rho(const float* x, const float* y, float* rho, int32_t nu
   cudaStream_t st = (cudaStream_t)stream;
   const int G = (int)G64;
   int* cnt = nullptr;
-  CK(cudaMallocAsync((void**)&cnt, (size_t)G * sizeof(int), st));
+  CK(scratch_alloc((void**)&cnt, (size_t)G * sizeof(int), st));
   CK(cudaMemsetAsync(cnt, 0, (size_t)G * sizeof(int), st));
   int g = (int)std::min<long>((num_p + 255) / 256, 148L * 16);
   k_count_cells<<<g, 256, 0, st>>>(x, y, nullptr, num_p, 0, cnt, nx, ny, (float)dx, (float)dy);
@@ -2023,9 +2167,9 @@ int32_t pb_compute_particle_substeps(const float* x, const float* y, const float
   const long long G = (long long)nx * ny;
   unsigned long long* bits = nullptr;
   float4* ec = nullptr;
-  CK(cudaMallocAsync((void**)&bits, 2 * sizeof(unsigned long long), st));
+  CK(scratch_alloc((void**)&bits, 2 * sizeof(unsigned long long), st));
   CK(cudaMemsetAsync(bits, 0, 2 * sizeof(unsigned long long), st));
-  CK(cudaMallocAsync((void**)&ec, (size_t)G * 2 * sizeof(float4), st));
+  CK(scratch_alloc((void**)&ec, (size_t)G * 2 * sizeof(float4), st));
   unsigned* ebound = reinterpret_cast<unsigned*>(bits + 1);
   const int gc = (int)std::min<long long>((G + 255) / 256, 148LL * 8);
   k_e_corners<<<gc, 256, 0, st>>>(Ex, Ey, ec, ny, nx, ebound);
