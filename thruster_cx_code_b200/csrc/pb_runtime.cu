@@ -2070,6 +2070,56 @@ int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float*
   return PB_OK;
 }
 
+// Where pb_accumulate_rho counts in shared-memory histograms (k_deposit_cluster) instead of
+// global atomics: up to DEPOSIT_ONE_MAX particles in one launch (two calls of 190k and 60k
+// particles take 35 us so and 36 us with the count kernels; at 100k and below the launches and
+// the scratch saved decide), and from DEPOSIT_MANY_MIN on, where the atomics on a small grid's
+// cells collide (two calls of 1.1M each on 65 x 284: 47 us; of 900k each by atomics 51 us).
+constexpr int DEPOSIT_ONE_MAX = 100000;
+constexpr int DEPOSIT_MANY_MIN = 1000000;
+constexpr int DEPOSIT_CLUSTERS = 18;   // of eight blocks: 144 SMs
+constexpr size_t DEPOSIT_CLUSTER_SMEM = 200 * 1024;
+static size_t deposit_smem(int G) { return ((size_t)G + 3) / 4 * 16; }
+
+// counts cleared, filled and rounded into rho
+static int32_t deposit_counts(const float* x, const float* y, float* rho, int num_p, double dx, double dy, int nx,
+                              int ny, double charge_density, int* cnt, cudaStream_t st, bool clusters) {
+  const int G = nx * ny;
+  CK(cudaMemsetAsync(cnt, 0, (size_t)G * sizeof(int), st));
+  if (clusters) {
+    k_deposit_cluster<<<DEPOSIT_CLUSTERS * DEP_C, 1024, deposit_smem(G), st>>>(x, y, rho, cnt, num_p, nx, ny, (float)dx, (float)dy,
+                                                                 charge_density);
+  } else {
+    const int g = (int)std::min<long>((num_p / 4 + 256) / 256, 148L * 8);
+    k_count_cells<<<g, 256, 0, st>>>(x, y, nullptr, num_p, 0, cnt, nx, ny, (float)dx, (float)dy);
+  }
+  CK(cudaGetLastError());
+  CK(launch_pdl(k_rho_finalize, (int)std::min<long>((G + 255) / 256, 148L * 16), 256, 0, st, rho, cnt, (int*)nullptr, G,
+                charge_density, 1));
+  return PB_OK;
+}
+
+// the kernel's shared-memory limit raised, once per context; false if it cannot be
+static bool deposit_cluster_ready() {
+  static std::mutex mu;
+  static unsigned long long seen[16] = {};
+  const unsigned long long id = current_context_id();
+  if (!id) return false;
+  std::lock_guard<std::mutex> lk(mu);
+  for (unsigned long long& s : seen) {
+    if (s == id) return true;
+    if (s) continue;
+    if (cudaFuncSetAttribute((const void*)k_deposit_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)DEPOSIT_CLUSTER_SMEM) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    s = id;
+    return true;
+  }
+  return false;
+}
+
 int32_t pb_accumulate_rho(const float* x, const float* y, float* rho, int32_t num_p, double dx, double dy, int32_t nx,
                           int32_t ny, double charge_density, void* stream) {
   if (nx < 3 || ny < 3) return fail(PB_ERR_ARG, "accumulate_rho: grid must be at least 3 x 3");
@@ -2079,15 +2129,19 @@ int32_t pb_accumulate_rho(const float* x, const float* y, float* rho, int32_t nu
   if (num_p <= 0) return PB_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const int G = (int)G64;
+  const bool clusters = G * sizeof(int) <= DEPOSIT_CLUSTER_SMEM && !stream_capturing(st) && deposit_cluster_ready();
+  if (clusters && num_p <= DEPOSIT_ONE_MAX) {
+    k_deposit_cluster<<<DEP_C, 1024, deposit_smem(G), st>>>(x, y, rho, nullptr, num_p, nx, ny, (float)dx, (float)dy,
+                                                            charge_density);
+    CK(cudaGetLastError());
+    return PB_OK;
+  }
   int* cnt = nullptr;
   CK(scratch_alloc((void**)&cnt, (size_t)G * sizeof(int), st));
-  CK(cudaMemsetAsync(cnt, 0, (size_t)G * sizeof(int), st));
-  int g = (int)std::min<long>((num_p + 255) / 256, 148L * 16);
-  k_count_cells<<<g, 256, 0, st>>>(x, y, nullptr, num_p, 0, cnt, nx, ny, (float)dx, (float)dy);
-  k_rho_finalize<<<(int)std::min<long>((G + 255) / 256, 148L * 16), 256, 0, st>>>(rho, cnt, nullptr, G,
-                                                                                  charge_density, 1);
-  CK(cudaFreeAsync(cnt, st));
-  CK(cudaGetLastError());
+  const int32_t rc = deposit_counts(x, y, rho, num_p, dx, dy, nx, ny, charge_density, cnt, st, clusters && num_p >= DEPOSIT_MANY_MIN);
+  const cudaError_t ef = cudaFreeAsync(cnt, st);
+  if (rc) return rc;
+  CK(ef);
   return PB_OK;
 }
 
@@ -2136,13 +2190,7 @@ int32_t pb_accumulate_rho_noalloc(const float* x, const float* y, float* rho, in
   // k_rho_finalize zeroes every count it reads, so after a call has completed the cells it
   // used are zero again.  This clear guards against a call that was cut off between its
   // two kernels (an error or a cancelled stream), which would leave counts behind.
-  CK(cudaMemsetAsync(cnt, 0, (size_t)G * sizeof(int), st));
-  int g = (int)std::min<long>((num_p + 255) / 256, 148L * 16);
-  k_count_cells<<<g, 256, 0, st>>>(x, y, nullptr, num_p, 0, cnt, nx, ny, (float)dx, (float)dy);
-  k_rho_finalize<<<(int)std::min<long>((G + 255) / 256, 148L * 16), 256, 0, st>>>(rho, cnt, nullptr, (int)G,
-                                                                                  charge_density, 1);
-  CK(cudaGetLastError());
-  return PB_OK;
+  return deposit_counts(x, y, rho, num_p, dx, dy, nx, ny, charge_density, cnt, st, false);
 }
 
 int32_t pb_thermal_conduction(const float* T, float* T_new, const int32_t* mask, int32_t nx, int32_t ny, double Fo_x,
