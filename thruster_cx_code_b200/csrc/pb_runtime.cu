@@ -2196,10 +2196,12 @@ int32_t pb_accumulate_rho_noalloc(const float* x, const float* y, float* rho, in
 int32_t pb_thermal_conduction(const float* T, float* T_new, const int32_t* mask, int32_t nx, int32_t ny, double Fo_x,
                               double Fo_y, void* stream) {
   if (nx < 1 || ny < 1) return fail(PB_ERR_ARG, "thermal_conduction: empty grid");
-  int G = nx * ny;
-  k_thermal_taichi<<<(int)std::min<long>((G + 255) / 256, 148L * 16), 256, 0, (cudaStream_t)stream>>>(
-      T, T_new, mask, nx, ny, (float)Fo_x, (float)Fo_y);
-  CK(cudaGetLastError());
+  const int G = nx * ny;
+  const bool vec = (((uintptr_t)T | (uintptr_t)T_new | (uintptr_t)mask) & 15u) == 0;
+  const int per = vec ? 4 : 1;
+  CK(launch_pdl(vec ? k_thermal_taichi<true> : k_thermal_taichi<false>,
+                (int)std::min<long>((G / per + 256) / 256, 148L * 16), 256, 0, (cudaStream_t)stream, T, T_new, mask, nx, ny,
+                (float)Fo_x, (float)Fo_y));
   return PB_OK;
 }
 
