@@ -240,6 +240,21 @@ PB_HD double philox_uniform(uint64_t seed, uint64_t pid, uint32_t site, uint32_t
 #define DDIV(a, b) ((a) / (b))
 #endif
 
+// RN(x / d) for an integer d < 2^40 and x = 0 or |x| >= 2^-900, with y = RN(1/d): one residual
+// correction of x y (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  x y is within 1.5 ulp of x / d and the residual is exact, so
+// the corrected value is x / d + e rounded once, |e| <= 2^-51 ulp, while x / d, not a midpoint,
+// is at least ulp / (2 d) away from one.  Three operations instead of a division's two dozen.
+PB_HD double div_int(double x, double d, double y) {
+#ifdef __CUDA_ARCH__
+  const double q = __dmul_rn(x, y);
+  return __fma_rn(__fma_rn(-q, d, x), y, q);
+#else
+  (void)y;
+  return x / d;
+#endif
+}
+
 PB_HD double bm_log(double x) {
   int e;
   double m = frexp(x, &e);
@@ -247,6 +262,9 @@ PB_HD double bm_log(double x) {
   double s = DDIV(DSUB(m, 1.0), DADD(m, 1.0));
   double s2 = DMUL(s, s);
   double acc = 1.0 / 27.0;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
   for (int k = 25; k >= 1; k -= 2) acc = DADD(DMUL(acc, s2), 1.0 / (double)k);
   return DADD(DMUL(DMUL(s, acc), 2.0), DMUL((double)e, 0.6931471805599453));
 }
@@ -260,8 +278,15 @@ PB_HD double bm_cos2pi(double u) {
   double r = DMUL(f, 0.7853981633974483);
   double r2 = DMUL(r, r);
   double c = 1.0, s = 1.0;
-  for (int n = 22; n >= 2; n -= 2) c = DSUB(1.0, DMUL(DDIV(r2, (double)(n * (n - 1))), c));
-  for (int n = 23; n >= 3; n -= 2) s = DSUB(1.0, DMUL(DDIV(r2, (double)(n * (n - 1))), s));
+  // r2 is 0 or at least 2^-108 (u is a multiple of 2^-53)
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int n = 22; n >= 2; n -= 2) c = DSUB(1.0, DMUL(div_int(r2, (double)(n * (n - 1)), 1.0 / (double)(n * (n - 1))), c));
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int n = 23; n >= 3; n -= 2) s = DSUB(1.0, DMUL(div_int(r2, (double)(n * (n - 1)), 1.0 / (double)(n * (n - 1))), s));
   s = DMUL(r, s);
   bool use_sin = (k == 1) | (k == 2) | (k == 5) | (k == 6);
   double v = use_sin ? s : c;

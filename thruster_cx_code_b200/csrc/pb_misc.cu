@@ -14,32 +14,41 @@ __device__ __forceinline__ int dep_cell(float x, float y, float dxf, float dyf, 
   return iy * nx + ix;
 }
 
-// Poisson(lam) by CDF inversion with one keyed uniform (oracle/philox.py: poisson_count)
+// Poisson(lam) by CDF inversion with one keyed uniform (oracle/philox.py: poisson_count), by a
+// warp: p_k = p_{k-1} lam / k is a chain of correctly rounded operations; its divisions by k
+// take reciprocals that the lanes form 32 at a time (div_int), four dependent operations a term
+// instead of a multiplication and a division.  Every lane returns the count.
 __device__ int poisson_inversion(double u, double lam) {
   if (!(lam > 0.0)) return 0;
+  const int lane = threadIdx.x & 31;
   double p = exp(-lam);
   double F = p;
   int k = 0;
-  int kmax = (int)(lam + 40.0 * sqrt(lam) + 100.0);
+  const int kmax = (int)(lam + 40.0 * sqrt(lam) + 100.0);
   while (u > F && k < kmax) {
-    ++k;
-    p = DDIV(DMUL(p, lam), (double)k);
-    F = DADD(F, p);
+    const double y = __drcp_rn((double)(k + 1 + lane));
+    for (int t = 0; t < 32 && u > F && k < kmax; ++t) {
+      ++k;
+      const double x = DMUL(p, lam), yk = __shfl_sync(0xFFFFFFFFu, y, t);
+      p = x >= 0x1p-900 ? div_int(x, (double)k, yk) : DDIV(x, (double)k);
+      F = DADD(F, p);
+    }
   }
   return k;
 }
 
 // ------------------------------------------------------------------ injection
-// inject step A (physics_engine.py:996-1099): counts, slots and ids for this step
-__global__ void k_inject_prep(InjectArgs a) {
+// inject step A (physics_engine.py:996-1099): counts, slots and ids for this step; one warp
+__global__ void __launch_bounds__(32) k_inject_prep(const __grid_constant__ InjectArgs a) {
   pdl_enter();
-  if (a.step_dev) a.step = *a.step_dev;
+  const uint32_t step = a.step_dev ? *a.step_dev : a.step;
   int n_ion = 0, n_rf = 0;
-  if (a.ion_on) n_ion = poisson_inversion(philox_uniform(a.seed, 0, SITE_ION_COUNT, a.step, 0), a.lam);
+  if (a.ion_on) n_ion = poisson_inversion(philox_uniform(a.seed, 0, SITE_ION_COUNT, step, 0), a.lam);
   if (a.rf_on) {
     n_rf = (int)a.rf_num_float;
-    if (philox_uniform(a.seed, 0, SITE_RF_COUNT, a.step, 0) < DSUB(a.rf_num_float, (double)n_rf)) ++n_rf;
+    if (philox_uniform(a.seed, 0, SITE_RF_COUNT, step, 0) < DSUB(a.rf_num_float, (double)n_rf)) ++n_rf;
   }
+  if (threadIdx.x != 0) return;
   int n_neut = a.neut_n;
   int np0 = *a.num_p, ne0 = *a.num_e;
   if (np0 + n_ion > a.cap_p) { atomicOr(a.errflags, PB_EF_CAPACITY_ION); n_ion = a.cap_p - np0; if (n_ion < 0) n_ion = 0; }
@@ -61,87 +70,78 @@ __global__ void k_inject_prep(InjectArgs a) {
   *a.next_e_id = id_e + n_rf + n_neut;
 }
 
-// inject step B: one thread per new particle; blockIdx.y selects ions / rf / neutralizer
-__global__ void k_inject_gen(InjectArgs a) {
+// inject step B: four threads per new particle (place, and one velocity component each);
+// blockIdx.y selects ions / rf / neutralizer.  The few particles make it a chain of latencies:
+// with three normals in sequence per thread, each of 24 float64 divisions, it held the step up
+// for 13 to 23 us on 130 x 568 and 26 us on 257 x 1025; 3 to 4 us so (div_int).
+__global__ void __launch_bounds__(128) k_inject_gen(const __grid_constant__ InjectArgs a) {
   pdl_enter();
-  if (a.step_dev) a.step = *a.step_dev;
+  const uint32_t step = a.step_dev ? *a.step_dev : a.step;
   const int seg = blockIdx.y;
   const int n = a.inj[seg];
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+  const int off = seg == 2 ? a.inj[1] : 0;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 4 * n; e += gridDim.x * blockDim.x) {
+    const int j = e >> 2, comp = (e & 3) - 1;
+    const uint32_t id = (uint32_t)a.inj[seg == 0 ? 5 : 6] + off + j;
+    const int slot = a.inj[seg == 0 ? 3 : 4] + off + j;
+    const Soa& S = seg == 0 ? a.ions : a.eles;
+    if (comp >= 0) {
+      const uint32_t site = seg == 0 ? SITE_ION_V : seg == 1 ? SITE_RF_V : SITE_NEUT_V;
+      const double g = philox_normal(a.seed, id, site, step, (uint32_t)comp);
+      double v;
+      if (seg == 0) v = comp == 0 ? DADD(a.v_bohm, DMUL(g, a.v_spread)) : DMUL(g, a.v_spread);
+      else if (seg == 1) v = comp == 0 ? DADD(DMUL(fabs(g), a.v_e_src), a.v_bohm) : DMUL(g, a.v_e_src);
+      else v = DMUL(g, a.v_e_th);
+      (comp == 0 ? S.vx : comp == 1 ? S.vy : S.vz)[slot] = __double2float_rn(v);
+      continue;
+    }
+    float x, y;
     if (seg == 0) {
-      uint32_t id = (uint32_t)a.inj[5] + j;
-      int slot = a.inj[3] + j;
-      float y;
       if (a.geometry == 2) {
-        double uh = philox_uniform(a.seed, id, SITE_ION_HOLE, a.step, 0);
-        double u = philox_uniform(a.seed, id, SITE_ION_HOLE, a.step, 1);
+        double uh = philox_uniform(a.seed, id, SITE_ION_HOLE, step, 0);
+        double u = philox_uniform(a.seed, id, SITE_ION_HOLE, step, 1);
         int which = (int)DMUL(uh, 2.0);
         float lo = a.span[2 * which], hi = a.span[2 * which + 1];
         y = __double2float_rn(DADD((double)lo, DMUL((double)__fsub_rn(hi, lo), u)));
       } else {
-        double u = philox_uniform(a.seed, id, SITE_ION_Y, a.step, 0);
+        double u = philox_uniform(a.seed, id, SITE_ION_Y, step, 0);
         y = __double2float_rn(DADD(a.ylo, DMUL(DSUB(a.yhi, a.ylo), u)));
       }
-      double g0 = philox_normal(a.seed, id, SITE_ION_V, a.step, 0);
-      double g1 = philox_normal(a.seed, id, SITE_ION_V, a.step, 1);
-      double g2 = philox_normal(a.seed, id, SITE_ION_V, a.step, 2);
-      float x = a.x_inj;
-      a.ions.x[slot] = x;
-      a.ions.y[slot] = y;
-      a.ions.vx[slot] = __double2float_rn(DADD(a.v_bohm, DMUL(g0, a.v_spread)));
-      a.ions.vy[slot] = __double2float_rn(DMUL(g1, a.v_spread));
-      a.ions.vz[slot] = __double2float_rn(DMUL(g2, a.v_spread));
-      a.ions.cex[slot] = 0;
-      a.ions.id[slot] = id;
-      atomicAdd(a.cnt_i + dep_cell(x, y, a.dxf, a.dyf, a.nx, a.ny), 1);
+      x = a.x_inj;
+      S.cex[slot] = 0;
+    } else if (seg == 1) {
+      double u = philox_uniform(a.seed, id, SITE_RF_Y, step, 0);
+      y = __double2float_rn(DADD(a.rf_ylo, DMUL(DSUB(a.rf_yhi, a.rf_ylo), u)));
+      x = 0.1f;
     } else {
-      bool rf = seg == 1;
-      int off = rf ? 0 : a.inj[1];
-      uint32_t id = (uint32_t)a.inj[6] + off + j;
-      int slot = a.inj[4] + off + j;
-      float x, y, vx, vy, vz;
-      if (rf) {
-        double u = philox_uniform(a.seed, id, SITE_RF_Y, a.step, 0);
-        y = __double2float_rn(DADD(a.rf_ylo, DMUL(DSUB(a.rf_yhi, a.rf_ylo), u)));
-        double g0 = philox_normal(a.seed, id, SITE_RF_V, a.step, 0);
-        double g1 = philox_normal(a.seed, id, SITE_RF_V, a.step, 1);
-        double g2 = philox_normal(a.seed, id, SITE_RF_V, a.step, 2);
-        x = 0.1f;
-        vx = __double2float_rn(DADD(DMUL(fabs(g0), a.v_e_src), a.v_bohm));
-        vy = __double2float_rn(DMUL(g1, a.v_e_src));
-        vz = __double2float_rn(DMUL(g2, a.v_e_src));
-      } else {
-        double u = philox_uniform(a.seed, id, SITE_NEUT_Y, a.step, 0);
-        y = __double2float_rn(DADD(0.0, DMUL(DSUB(a.neut_r, 0.0), u)));
-        double g0 = philox_normal(a.seed, id, SITE_NEUT_V, a.step, 0);
-        double g1 = philox_normal(a.seed, id, SITE_NEUT_V, a.step, 1);
-        double g2 = philox_normal(a.seed, id, SITE_NEUT_V, a.step, 2);
-        x = a.neut_x;
-        vx = __double2float_rn(DMUL(g0, a.v_e_th));
-        vy = __double2float_rn(DMUL(g1, a.v_e_th));
-        vz = __double2float_rn(DMUL(g2, a.v_e_th));
-      }
-      a.eles.x[slot] = x; a.eles.y[slot] = y;
-      a.eles.vx[slot] = vx; a.eles.vy[slot] = vy; a.eles.vz[slot] = vz;
-      a.eles.id[slot] = id;
-      atomicAdd(a.cnt_e + dep_cell(x, y, a.dxf, a.dyf, a.nx, a.ny), 1);
+      double u = philox_uniform(a.seed, id, SITE_NEUT_Y, step, 0);
+      y = __double2float_rn(DADD(0.0, DMUL(DSUB(a.neut_r, 0.0), u)));
+      x = a.neut_x;
     }
+    S.x[slot] = x;
+    S.y[slot] = y;
+    S.id[slot] = id;
+    atomicAdd((seg == 0 ? a.cnt_i : a.cnt_e) + dep_cell(x, y, a.dxf, a.dyf, a.nx, a.ny), 1);
   }
 }
 
 // ------------------------------------------------------------------ single-block bitonic sort
-// Sorts keys[0..n) ascending in place (global memory; one block, any n <= cap).
-__device__ void block_sort_u64(uint64_t* keys, int n) {
+// Sorts keys[0..n) ascending in place (one block; shared memory, or global memory with room for
+// the next power of two).  Each of the log^2 steps of a short list costs a barrier in shared
+// memory but a round trip to L2 in global memory, so lists of up to SORT_SMEM keys are copied.
+constexpr int SORT_SMEM = 2048;
+template <class T>
+__device__ __forceinline__ void block_sort(T* keys, int n) {
   int m = 1;
   while (m < n) m <<= 1;
-  for (int i = n + threadIdx.x; i < m; i += blockDim.x) keys[i] = ~0ull;
+  for (int i = n + threadIdx.x; i < m; i += blockDim.x) keys[i] = (T)~(T)0;
   __syncthreads();
   for (int k = 2; k <= m; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
       for (int i = threadIdx.x; i < m; i += blockDim.x) {
         int l = i ^ j;
         if (l > i) {
-          uint64_t a = keys[i], b = keys[l];
+          T a = keys[i], b = keys[l];
           bool up = (i & k) == 0;
           if ((a > b) == up) { keys[i] = b; keys[l] = a; }
         }
@@ -155,31 +155,43 @@ __device__ void block_sort_u64(uint64_t* keys, int n) {
 // Spawned electrons in parent-id order (= the reference's array order), keyed draws by
 // the parent ion, purge test against the current isBound, appended after the step's
 // surviving electrons (physics_engine.py:1400-1417, 1541-1561).
-__global__ void k_see_finish(SeeArgs a) {
+__global__ void __launch_bounds__(1024) k_see_finish(const __grid_constant__ SeeArgs a) {
   pdl_enter();
-  if (a.step_dev) a.step = *a.step_dev;
+  const uint32_t step = a.step_dev ? *a.step_dev : a.step;
   __shared__ int sm[32];
   __shared__ int s_base, s_total;
+  __shared__ uint64_t skey[SORT_SMEM];
+  __shared__ float svel[3 * 1024];
   int n = *a.see_count;
   if (n > a.see_cap) n = a.see_cap;
-  block_sort_u64(a.see_key, n);
+  const bool small = n <= SORT_SMEM;
+  uint64_t* const keys = small ? skey : a.see_key;
+  if (small) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) skey[i] = a.see_key[i];
+    __syncthreads();
+    block_sort(skey, n);
+  } else {
+    block_sort(a.see_key, n);
+  }
   const int ne0 = *a.num_e;
   const uint32_t id0 = *a.next_e_id;
   int done = 0;
   for (int c0 = 0; c0 < n; c0 += blockDim.x) {
+    // the chunk's velocity components, one per thread and turn
+    const int nc = min(n - c0, (int)blockDim.x);
+    for (int e = threadIdx.x; e < 3 * nc; e += blockDim.x) {
+      const uint32_t parent = (uint32_t)(keys[c0 + e / 3] >> 32);
+      svel[e] = __double2float_rn(DMUL(philox_normal(a.seed, parent, SITE_SEE_V, step, (uint32_t)(e % 3)), a.v_see_th));
+    }
+    __syncthreads();
     int r = c0 + threadIdx.x;
     bool keep = false;
     float x = 0, y = 0, vx = 0, vy = 0, vz = 0;
-    uint32_t parent = 0;
     if (r < n) {
-      uint64_t key = a.see_key[r];
-      parent = (uint32_t)(key >> 32);
-      uint32_t rec = (uint32_t)key;
+      const uint32_t rec = (uint32_t)keys[r];
       x = a.see_xy[2 * rec];
       y = a.see_xy[2 * rec + 1];
-      vx = __double2float_rn(DMUL(philox_normal(a.seed, parent, SITE_SEE_V, a.step, 0), a.v_see_th));
-      vy = __double2float_rn(DMUL(philox_normal(a.seed, parent, SITE_SEE_V, a.step, 1), a.v_see_th));
-      vz = __double2float_rn(DMUL(philox_normal(a.seed, parent, SITE_SEE_V, a.step, 2), a.v_see_th));
+      vx = svel[3 * threadIdx.x]; vy = svel[3 * threadIdx.x + 1]; vz = svel[3 * threadIdx.x + 2];
       int icx = cell_round(x, a.dxf, 0, a.nx - 1), icy = cell_round(y, a.dyf, 0, a.ny - 1);
       bool dead = a.isBound[(size_t)icy * a.nx + icx] != 0;
       dead = dead || (x < 0.0f) || (x > a.Lxf) || (y < 0.0f) || (y > a.Lyf) || (x != x);
@@ -243,9 +255,17 @@ __global__ void k_theta95(float* angles, const int* count, int cap, uint64_t* sc
     if (threadIdx.x == 0) *out = __longlong_as_double(0x7ff8000000000000ll);
     return;
   }
+  if (n <= 2 * SORT_SMEM) {
+    __shared__ uint32_t skey[2 * SORT_SMEM];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) skey[i] = __float_as_uint(angles[i]);
+    __syncthreads();
+    block_sort(skey, n);
+    if (threadIdx.x == 0) *out = (double)percentile95_sorted(reinterpret_cast<const float*>(skey), n);
+    return;
+  }
   for (int i = threadIdx.x; i < n; i += blockDim.x) scratch[i] = (uint64_t)__float_as_uint(angles[i]);
   __syncthreads();
-  block_sort_u64(scratch, n);
+  block_sort(scratch, n);
   for (int i = threadIdx.x; i < n; i += blockDim.x) angles[i] = __uint_as_float((uint32_t)scratch[i]);
   __syncthreads();
   if (threadIdx.x == 0) *out = (double)percentile95_sorted(angles, n);
@@ -310,29 +330,41 @@ __global__ void k_refresh_dinv0(const uint8_t* cls, float* dinv, int ny, int nx,
 // Radiative cooling of bound cells, 10 explicit FTCS sweeps over interior bound cells
 // (non-bound neighbours replaced by the centre value, T_new = max(T + dT, 300)) and the
 // final clamp, fused with temporal blocking: each block owns a TT x TT output tile and
-// loads a halo of SWEEPS cells (physics_engine.py:1566-1615, CPU-loop semantics).
+// loads a halo of SWEEPS cells (physics_engine.py:1566-1615, CPU-loop semantics).  The bound
+// cells' new temperatures go to Tnext (other blocks' halos are still to be read from T);
+// k_grid_sums moves them.
+// A thread keeps its cells' values, neighbour tests and indexes in registers over the sweeps;
+// 1024 threads (three cells each), since a small grid has few tiles (27 on 65 x 284) and a sweep
+// is latency: that grid's step took 19.5 us for it with 256 threads that indexed every cell of
+// every sweep, 7.1 us so.
 constexpr int TT = 32;
 constexpr int HALO = 10;
 constexpr int TW = TT + 2 * HALO;
+constexpr int THERMAL_NT = 1024;
 
-__global__ void __launch_bounds__(256) k_thermal(float* T, const uint8_t* isBound, int ny, int nx, float cf,
-                                                 float T4_300, float Fo_x, float Fo_y, int sweeps) {
+__global__ void __launch_bounds__(THERMAL_NT) k_thermal(const float* T, float* Tnext, const uint8_t* isBound, int ny,
+                                                        int nx, float cf, float T4_300, float Fo_x, float Fo_y,
+                                                        int sweeps) {
   pdl_enter();
-  __shared__ float A[TW * TW], B[TW * TW];
+  constexpr int PER = (TW * TW + THERMAL_NT - 1) / THERMAL_NT;
+  __shared__ float buf[2][TW * TW];
   __shared__ uint8_t M[TW * TW];
-  __shared__ int any;
   const int gx0 = blockIdx.x * TT - HALO, gy0 = blockIdx.y * TT - HALO;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
+  float c[PER];
+  unsigned flags[PER];  // bits 0-3: the neighbour left, right, down, up is bound; 4: swept; 5: bound; 6: output
   int found = 0;
-  for (int k = threadIdx.x; k < TW * TW; k += blockDim.x) {
-    int ly = k / TW, lx = k - ly * TW;
-    int gy = gy0 + ly, gx = gx0 + lx;
-    bool in = gy >= 0 && gy < ny && gx >= 0 && gx < nx;
-    float t = 0.0f;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int k = threadIdx.x + j * THERMAL_NT;
+    c[j] = 0.0f;
+    flags[j] = 0u;
+    if (k >= TW * TW) continue;
+    const int ly = k / TW, lx = k - ly * TW;
+    const int gy = gy0 + ly, gx = gx0 + lx;
+    const bool in = gy >= 0 && gy < ny && gx >= 0 && gx < nx;
     uint8_t m = 0;
     if (in) {
-      t = T[(size_t)gy * nx + gx];
+      float t = T[(size_t)gy * nx + gx];
       m = isBound[(size_t)gy * nx + gx];
       if (m) {
         // T -= cf * (T**4 - 300**4)   (x^4 rounded once from double)
@@ -341,47 +373,53 @@ __global__ void __launch_bounds__(256) k_thermal(float* T, const uint8_t* isBoun
         t = __fsub_rn(t, __fmul_rn(cf, __fsub_rn(t4, T4_300)));
         found = 1;
       }
+      c[j] = t;
+      if (m & 1) flags[j] |= 32u;
+      if ((m & 1) && gy >= 1 && gy <= ny - 2 && gx >= 1 && gx <= nx - 2 && ly >= 1 && ly <= TW - 2 && lx >= 1 &&
+          lx <= TW - 2)
+        flags[j] |= 16u;
+      if (ly >= HALO && ly < HALO + TT && lx >= HALO && lx < HALO + TT) flags[j] |= 64u;
     }
-    A[k] = t;
-    M[k] = m | (in ? 2 : 0);
+    buf[0][k] = c[j];
+    M[k] = m;
   }
-  if (found) any = 1;
-  __syncthreads();
-  if (!any) return;
-  float* cur = A;
-  float* nxt = B;
+  if (!__syncthreads_or(found)) return;
+#pragma unroll
+  for (int j = 0; j < PER; ++j)
+    if (flags[j] & 16u) {
+      const int k = threadIdx.x + j * THERMAL_NT;
+      flags[j] |= (M[k - 1] & 1u) | (M[k + 1] & 1u) << 1 | (M[k - TW] & 1u) << 2 | (M[k + TW] & 1u) << 3;
+    }
   for (int s = 0; s < sweeps; ++s) {
-    for (int k = threadIdx.x; k < TW * TW; k += blockDim.x) {
-      int ly = k / TW, lx = k - ly * TW;
-      int gy = gy0 + ly, gx = gx0 + lx;
-      float c = cur[k];
-      float v = c;
-      bool upd = (M[k] & 1) && gy >= 1 && gy <= ny - 2 && gx >= 1 && gx <= nx - 2 && ly >= 1 && ly <= TW - 2 &&
-                 lx >= 1 && lx <= TW - 2;
-      if (upd) {
-        float tl = (M[k - 1] & 1) ? cur[k - 1] : c;
-        float tr = (M[k + 1] & 1) ? cur[k + 1] : c;
-        float td = (M[k - TW] & 1) ? cur[k - TW] : c;
-        float tu = (M[k + TW] & 1) ? cur[k + TW] : c;
-        float c2 = __fmul_rn(2.0f, c);
-        float dT = __fadd_rn(__fmul_rn(Fo_x, __fadd_rn(__fsub_rn(tl, c2), tr)),
-                             __fmul_rn(Fo_y, __fadd_rn(__fsub_rn(td, c2), tu)));
-        float nv = __fadd_rn(c, dT);
-        v = (nv != nv) ? nv : (nv > 300.0f ? nv : 300.0f);
+    const float* cur = buf[s & 1];
+    float* nxt = buf[(s & 1) ^ 1];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int k = threadIdx.x + j * THERMAL_NT;
+      if (k >= TW * TW) continue;
+      if (flags[j] & 16u) {
+        const float v = c[j];
+        const float tl = flags[j] & 1u ? cur[k - 1] : v;
+        const float tr = flags[j] & 2u ? cur[k + 1] : v;
+        const float td = flags[j] & 4u ? cur[k - TW] : v;
+        const float tu = flags[j] & 8u ? cur[k + TW] : v;
+        const float c2 = __fmul_rn(2.0f, v);
+        const float dT = __fadd_rn(__fmul_rn(Fo_x, __fadd_rn(__fsub_rn(tl, c2), tr)),
+                                   __fmul_rn(Fo_y, __fadd_rn(__fsub_rn(td, c2), tu)));
+        const float nv = __fadd_rn(v, dT);
+        c[j] = (nv != nv) ? nv : (nv > 300.0f ? nv : 300.0f);
       }
-      nxt[k] = v;
+      nxt[k] = c[j];
     }
     __syncthreads();
-    float* t = cur; cur = nxt; nxt = t;
   }
-  for (int k = threadIdx.x; k < TW * TW; k += blockDim.x) {
-    int ly = k / TW, lx = k - ly * TW;
-    if (ly < HALO || ly >= HALO + TT || lx < HALO || lx >= HALO + TT) continue;
-    int gy = gy0 + ly, gx = gx0 + lx;
-    if (gy >= ny || gx >= nx) continue;
-    float v = cur[k];
-    if (M[k] & 1) v = (v != v) ? v : (v > 300.0f ? v : 300.0f);
-    T[(size_t)gy * nx + gx] = v;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    if ((flags[j] & 96u) != 96u) continue;
+    const int k = threadIdx.x + j * THERMAL_NT;
+    const int ly = k / TW, lx = k - ly * TW;
+    const float v = c[j];
+    Tnext[(size_t)(gy0 + ly) * nx + gx0 + lx] = (v != v) ? v : (v > 300.0f ? v : 300.0f);
   }
 }
 
@@ -403,15 +441,18 @@ __device__ __forceinline__ T block_reduce(T v, Op op, T ident) {
   return v;
 }
 
-__global__ void k_grid_sums(const float* T, const uint16_t* gridmask, int N, int ngrids, double* out) {
+// With Tnext, the bound cells' new temperatures from k_thermal are moved into T first.
+__global__ void k_grid_sums(float* T, const float* Tnext, const uint8_t* isBound, const uint16_t* gridmask, int N,
+                            int ngrids, double* out) {
   pdl_enter();
   double s[16];
   double c[16];
   for (int g = 0; g < ngrids; ++g) { s[g] = 0; c[g] = 0; }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    uint16_t m = gridmask[i];
+    const uint16_t m = gridmask[i];
+    if (Tnext && isBound[i]) T[i] = Tnext[i];
     if (!m) continue;
-    double t = (double)T[i];
+    const double t = (double)T[i];
     for (int g = 0; g < ngrids; ++g)
       if (m & (1u << g)) { s[g] += t; c[g] += 1.0; }
   }

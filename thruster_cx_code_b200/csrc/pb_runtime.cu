@@ -173,7 +173,7 @@ struct Sim {
   int ny = 0, nx = 0, periodic = 0, ngrids = 0;
   double *V = nullptr, *Vnew = nullptr, *Vfixed = nullptr, *Vdc = nullptr, *damage = nullptr, *eroded = nullptr;
   double *accum_ppc = nullptr, *f = nullptr, *dirsum = nullptr;
-  float *Ex = nullptr, *Ey = nullptr, *rho = nullptr, *Tmap = nullptr;
+  float *Ex = nullptr, *Ey = nullptr, *rho = nullptr, *Tmap = nullptr, *Tnext = nullptr;
   float *r32 = nullptr, *z32 = nullptr, *p32 = nullptr, *q32 = nullptr, *e32 = nullptr;
   float *s32 = nullptr, *m32 = nullptr;  // fine-level smoothing temporaries (nu = 2)
   float4* ecorn = nullptr;  // per-cell corners of Ex and Ey, 2 x float4 per node
@@ -705,8 +705,9 @@ struct SaddleIdx { int v[8]; };
 // eight saddle nodes; 0 without any) and the solver statistics, in one thread.
 __global__ void k_report(pb_step_report* r, const int* counts, int ci, int ce, const int* n_sub,
                          const unsigned long long* ds_bits, const int* inj, const int* see_spawned, const double* V,
-                         int n_saddle, SaddleIdx sidx, const double* pstats) {
+                         int n_saddle, SaddleIdx sidx, const double* pstats, const uint32_t* mg_status) {
   pdl_enter();
+  *reinterpret_cast<uint32_t*>(r + 1) = *mg_status;  // past the report: one copy brings both to the host
   r->num_p = counts[ci];
   r->num_e = counts[2 + ce];
   r->n_sub_ion = n_sub[0];
@@ -914,12 +915,12 @@ static int32_t enqueue_step_pre(pb_sim* h, const pb_step_params* p) {
   ia.ions = I.buf[I.cur]; ia.eles = E.buf[E.cur];
   ia.cnt_i = s->cnt_i; ia.cnt_e = s->cnt_e;
   ia.nx = s->nx; ia.ny = s->ny; ia.dxf = dxf; ia.dyf = dyf; ia.errflags = ef;
-  CK(launch_pdl(k_inject_prep, 1, 1, 0, st, ia));
+  CK(launch_pdl(k_inject_prep, 1, 32, 0, st, ia));
   ++s->launches;
   {
     long mx = std::max<long>({(long)(p->lam + 40.0 * std::sqrt(std::max(p->lam, 0.0)) + 100.0),
                               (long)p->neut_n, (long)p->rf_num_float + 1, 1L});
-    CK(launch_pdl(k_inject_gen, dim3(grid_for(s, mx, 128, 2), 3), 128, 0, st, ia));
+    CK(launch_pdl(k_inject_gen, dim3(grid_for(s, 4 * mx, 128, 4), 3), 128, 0, st, ia));
     ++s->launches;
   }
 
@@ -1061,14 +1062,14 @@ static int32_t enqueue_step_post(pb_sim* h, const pb_step_params* p) {
 
   // F. thermal (:1566-1620)
   if (p->thermal_on) {
-    CK(launch_pdl(k_thermal, dim3((s->nx + TT - 1) / TT, (s->ny + TT - 1) / TT), 256, 0, st,
-        s->Tmap, s->isBound, s->ny, s->nx, (float)p->cooling_factor, (float)p->T4_300, (float)p->Fo_x,
+    CK(launch_pdl(k_thermal, dim3((s->nx + TT - 1) / TT, (s->ny + TT - 1) / TT), THERMAL_NT, 0, st,
+        s->Tmap, s->Tnext, s->isBound, s->ny, s->nx, (float)p->cooling_factor, (float)p->T4_300, (float)p->Fo_x,
         (float)p->Fo_y, p->sweeps));
     ++s->launches;
   }
-  if (s->ngrids > 0) {
-    CK(launch_pdl(k_grid_sums, grid_for(s, N, 256), 256, 0, st, s->Tmap, s->gridmask, N, std::min(s->ngrids, 16),
-                  rep->grid_sums));
+  if (s->ngrids > 0 || p->thermal_on) {
+    CK(launch_pdl(k_grid_sums, grid_for(s, N, 256), 256, 0, st, s->Tmap, p->thermal_on ? s->Tnext : nullptr, s->isBound,
+                  s->gridmask, N, std::min(s->ngrids, 16), rep->grid_sums));
     ++s->launches;
   }
   mark(s);
@@ -1079,7 +1080,7 @@ static int32_t enqueue_step_post(pb_sim* h, const pb_step_params* p) {
   SaddleIdx sidx{};
   for (int k = 0; k < 8; ++k) sidx.v[k] = p->saddle_idx[k];
   CK(launch_pdl(k_report, 1, 1, 0, st, rep, s->counts, I.cur, E.cur, s->n_sub, s->ds_bits, s->inj, s->see_spawned, s->V,
-                            std::max(0, std::min(p->n_saddle, 8)), sidx, s->pstats));
+                            std::max(0, std::min(p->n_saddle, 8)), sidx, s->pstats, s->mg_status));
   ++s->launches;
   CK(launch_pdl(k_ppc_stats, grid_for(s, N, 256), 256, 0, st, s->ppc, s->accum_ppc, N,
                 (unsigned long long*)&rep->ppc_active));
@@ -1137,7 +1138,7 @@ static uint64_t state_signature(const pb_sim* h) {
     for (int b = 0; b < 2; ++b) k = fnv_v(k, S.buf[b]);
   }
   const void* ptrs[] = {s->V, s->Vnew, s->Vfixed, s->Vdc, s->damage, s->eroded, s->accum_ppc, s->f, s->dirsum,
-                        s->Ex, s->Ey, s->rho, s->Tmap, s->r32, s->z32, s->p32, s->q32, s->e32, s->s32, s->m32,
+                        s->Ex, s->Ey, s->rho, s->Tmap, s->Tnext, s->r32, s->z32, s->p32, s->q32, s->e32, s->s32, s->m32,
                         s->ecorn,
                         s->isBound, s->cls, s->bdist, s->gridmask, s->ppc, s->cnt_i, s->cnt_e, s->cidx, s->cinv,
                         s->partials, s->bar, s->pstats, s->ptrace, s->counts, s->next_ids, s->tile_status,
@@ -1261,10 +1262,13 @@ static int32_t run_one_step(pb_sim* h, const pb_step_params* p) {
   return enqueue_step(h, p);
 }
 
-static int32_t finish_report(Sim* s, pb_step_report* out) {
-  CK(cudaMemcpyAsync(s->rep_host, s->rep_dev, sizeof(pb_step_report), cudaMemcpyDeviceToHost, s->stream));
+// the report and, past it, the rebuild's status (k_report)
+static int32_t finish_report(Sim* s, pb_step_report* out, uint32_t* mg_status) {
+  CK(cudaMemcpyAsync(s->rep_host, s->rep_dev, sizeof(pb_step_report) + sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                     s->stream));
   CK(cudaStreamSynchronize(s->stream));
   *out = *s->rep_host;
+  std::memcpy(mg_status, s->rep_host + 1, sizeof(uint32_t));
   s->host_num[0] = out->num_p;
   s->host_num[1] = out->num_e;
   return check_flags(s, out->errflags);
@@ -1316,11 +1320,11 @@ int32_t pb_sim_create(pb_sim** out, int32_t device) {
   CK(dalloc(&s->see_xy, 2 * (size_t)s->see_cap));
   CK(dalloc(&s->angles, (size_t)s->angle_cap));
   CK(dalloc(&s->angle_scratch, 2 * (size_t)s->angle_cap));
-  CK(dalloc(&s->rep_dev, 1));
-  CK(cudaMemset(s->rep_dev, 0, sizeof(pb_step_report)));
+  CK(dalloc(&s->rep_dev, 2));  // the report and the words past it (k_report)
+  CK(cudaMemset(s->rep_dev, 0, 2 * sizeof(pb_step_report)));
   CK(dalloc(&s->step_dev, 1));
   CK(cudaMemset(s->step_dev, 0, sizeof(uint32_t)));
-  CK(cudaMallocHost((void**)&s->rep_host, sizeof(pb_step_report)));
+  CK(cudaMallocHost((void**)&s->rep_host, 2 * sizeof(pb_step_report)));
   s->sp[0].ion = true;
   s->sp[1].ion = false;
   CK(cudaEventCreate(&s->ev0));
@@ -1342,7 +1346,7 @@ int32_t pb_sim_destroy(pb_sim* h) {
   free_levels(s);
   double* d[] = {s->V, s->Vnew, s->Vfixed, s->Vdc, s->damage, s->eroded, s->accum_ppc, s->f, s->dirsum, s->partials, s->pstats};
   for (double* q : d) if (q) cudaFree(q);
-  float* fl[] = {s->Ex, s->Ey, s->rho, s->Tmap, s->r32, s->z32, s->p32, s->q32, s->e32, s->s32, s->m32,
+  float* fl[] = {s->Ex, s->Ey, s->rho, s->Tmap, s->Tnext, s->r32, s->z32, s->p32, s->q32, s->e32, s->s32, s->m32,
                  s->see_xy, s->angles};
   for (float* q : fl) if (q) cudaFree(q);
   if (s->ecorn) cudaFree(s->ecorn);
@@ -1468,7 +1472,7 @@ int32_t pb_sim_set_domain(pb_sim* h, int32_t ny, int32_t nx, int32_t periodic, c
     if (keep_state && s->domain_set) return fail(PB_ERR_ARG, "pb_sim_set_domain: keep_state with a new grid size");
     double** dd[] = {&s->V, &s->Vnew, &s->Vfixed, &s->Vdc, &s->damage, &s->eroded, &s->accum_ppc, &s->f, &s->dirsum};
     for (double** q : dd) { dfree(*q); CK(dalloc(q, N)); CK(cudaMemset(*q, 0, N * sizeof(double))); }
-    float** ff[] = {&s->Ex, &s->Ey, &s->rho, &s->Tmap, &s->r32, &s->z32, &s->p32, &s->q32, &s->e32, &s->s32,
+    float** ff[] = {&s->Ex, &s->Ey, &s->rho, &s->Tmap, &s->Tnext, &s->r32, &s->z32, &s->p32, &s->q32, &s->e32, &s->s32,
                     &s->m32};
     for (float** q : ff) { dfree(*q); CK(dalloc(q, N)); CK(cudaMemset(*q, 0, N * sizeof(float))); }
     dfree(s->ecorn); CK(dalloc(&s->ecorn, 2 * N)); CK(cudaMemset(s->ecorn, 0, 2 * N * sizeof(float4)));
@@ -1513,11 +1517,16 @@ int32_t pb_sim_set_domain(pb_sim* h, int32_t ny, int32_t nx, int32_t periodic, c
 
 // After a run: a break whose freed nodes change the level structure was left to the host
 // by k_mg_rebuild (MG_STATUS_HOST); rebuild the hierarchy here before the next solve.
-static int32_t settle_mg(Sim* s) {
+// status: the rebuild's status when the caller has read it with a step report.
+static int32_t settle_mg(Sim* s, const uint32_t* status = nullptr) {
   if (!s->erosion_seen || !s->mg_status) return PB_OK;
   uint32_t st = 0;
-  CK(cudaMemcpyAsync(&st, s->mg_status, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaStreamSynchronize(s->stream));
+  if (status) {
+    st = *status;
+  } else {
+    CK(cudaMemcpyAsync(&st, s->mg_status, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+  }
   if (!(st & MG_STATUS_HOST)) return PB_OK;
   std::vector<uint8_t> ib((size_t)s->ny * s->nx);
   CK(cudaMemcpy(ib.data(), s->isBound, ib.size(), cudaMemcpyDeviceToHost));
@@ -1712,11 +1721,12 @@ int32_t pb_sim_step(pb_sim* h, const pb_step_params* p, pb_step_report* report) 
   if ((rc = run_one_step(h, p))) return rc;
   CK(cudaEventRecord(s->ev1, s->stream));
   if (report) {
-    if ((rc = finish_report(s, report))) return rc;
+    uint32_t status = 0;
+    if ((rc = finish_report(s, report, &status))) return rc;
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
     s->last_ms = ms;
-    if ((rc = settle_mg(s))) return rc;
+    if ((rc = settle_mg(s, &status))) return rc;
   }
   return PB_OK;
 }
