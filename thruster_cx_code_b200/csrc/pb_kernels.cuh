@@ -122,6 +122,20 @@ struct IonStepArgs {
   uint32_t *errflags;
 };
 
+// The sub-step reductions of both species (k_substep_both); index 0: ions
+struct SubstepArgs {
+  Soa sp[2];
+  const int *n[2];
+  double qm[2];
+  const float4* Ec;
+  const unsigned* ebound;
+  int nx, ny;
+  float dxf, dyf, dtf;
+  double dt2;
+  unsigned long long* ds_max_bits;
+  int ion_blocks;
+};
+
 struct EleStepArgs {
   Soa src, dst;
   const int *num_src;

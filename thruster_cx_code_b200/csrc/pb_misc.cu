@@ -39,8 +39,8 @@ __device__ int poisson_inversion(double u, double lam) {
 
 // ------------------------------------------------------------------ injection
 // inject step A (physics_engine.py:996-1099): counts, slots and ids for this step; one warp
-__global__ void __launch_bounds__(32) k_inject_prep(const __grid_constant__ InjectArgs a) {
-  pdl_enter();
+// (of k_step_reset)
+__device__ __forceinline__ void inject_counts(const InjectArgs& a) {
   const uint32_t step = a.step_dev ? *a.step_dev : a.step;
   int n_ion = 0, n_rf = 0;
   if (a.ion_on) n_ion = poisson_inversion(philox_uniform(a.seed, 0, SITE_ION_COUNT, step, 0), a.lam);
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(32) k_inject_prep(const __grid_constant__ Inje
     n_rf = (int)a.rf_num_float;
     if (philox_uniform(a.seed, 0, SITE_RF_COUNT, step, 0) < DSUB(a.rf_num_float, (double)n_rf)) ++n_rf;
   }
-  if (threadIdx.x != 0) return;
+  if ((threadIdx.x & 31) != 0) return;
   int n_neut = a.neut_n;
   int np0 = *a.num_p, ne0 = *a.num_e;
   if (np0 + n_ion > a.cap_p) { atomicOr(a.errflags, PB_EF_CAPACITY_ION); n_ion = a.cap_p - np0; if (n_ion < 0) n_ion = 0; }
@@ -247,8 +247,7 @@ PB_HD float percentile95_sorted(const float* s, int n) {
   return g >= 0.5f ? hi - d * (1.0f - g) : lo + d * g;
 }
 
-__global__ void k_theta95(float* angles, const int* count, int cap, uint64_t* scratch, double* out) {
-  pdl_enter();
+__device__ void theta95(float* angles, const int* count, int cap, uint64_t* scratch, double* out) {
   int n = *count;
   if (n > cap) n = cap;
   if (n <= 5) {
@@ -332,7 +331,7 @@ __global__ void k_refresh_dinv0(const uint8_t* cls, float* dinv, int ny, int nx,
 // final clamp, fused with temporal blocking: each block owns a TT x TT output tile and
 // loads a halo of SWEEPS cells (physics_engine.py:1566-1615, CPU-loop semantics).  The bound
 // cells' new temperatures go to Tnext (other blocks' halos are still to be read from T);
-// k_grid_sums moves them.
+// node_stats moves them.
 // A thread keeps its cells' values, neighbour tests and indexes in registers over the sweeps;
 // 1024 threads (three cells each), since a small grid has few tiles (27 on 65 x 284) and a sweep
 // is latency: that grid's step took 19.5 us for it with 256 threads that indexed every cell of
@@ -423,7 +422,6 @@ __global__ void __launch_bounds__(THERMAL_NT) k_thermal(const float* T, float* T
   }
 }
 
-// grid means over each electrode mask (bit g of gridmask) -> sums[2g], counts[2g+1]
 // Block-wide reduction with op; the result is valid in thread 0.  Ends with a barrier, so
 // it can be called again at once.  blockDim.x is a multiple of 32.
 template <class T, class Op>
@@ -441,48 +439,52 @@ __device__ __forceinline__ T block_reduce(T v, Op op, T ident) {
   return v;
 }
 
-// With Tnext, the bound cells' new temperatures from k_thermal are moved into T first.
-__global__ void k_grid_sums(float* T, const float* Tnext, const uint8_t* isBound, const uint16_t* gridmask, int N,
-                            int ngrids, double* out) {
-  pdl_enter();
-  double s[16];
-  double c[16];
-  for (int g = 0; g < ngrids; ++g) { s[g] = 0; c[g] = 0; }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    const uint16_t m = gridmask[i];
-    if (Tnext && isBound[i]) T[i] = Tnext[i];
-    if (!m) continue;
-    const double t = (double)T[i];
-    for (int g = 0; g < ngrids; ++g)
-      if (m & (1u << g)) { s[g] += t; c[g] += 1.0; }
-  }
-  // one pair of atomics per block and grid (per-warp atomics on the same 2 * ngrids
-  // words serialised at L2)
-  const auto add = [](double a, double b) { return a + b; };
-  for (int g = 0; g < ngrids; ++g) {
-    const double a = block_reduce(s[g], add, 0.0), b = block_reduce(c[g], add, 0.0);
-    if (threadIdx.x == 0 && b != 0.0) { atomicAdd(out + 2 * g, a); atomicAdd(out + 2 * g + 1, b); }
-  }
-}
+// One pass over the nodes, block `block` of `blocks`: the bound cells' new temperatures from
+// k_thermal moved into T (Tnext not null), the electrodes' sums, and the PPC statistics: accum
+// += ppc; total active cells, cells with 0 < ppc < 3, min nonzero.
+constexpr int STEP_END_NT = 512;
 
-// ------------------------------------------------------------------ PPC statistics
-// accum += ppc; total active cells, cells with 0 < ppc < 3, min nonzero
-__global__ void k_ppc_stats(const int* ppc, double* accum, int N, unsigned long long* stats) {
-  pdl_enter();
-  unsigned long long act = 0, low = 0;
+__device__ __forceinline__ void node_stats(float* T, const float* Tnext, const uint8_t* isBound,
+                                           const uint16_t* gridmask, int ngrids, double* sums, const int* ppc,
+                                           double* accum, unsigned long long* stats, int N, int block, int blocks) {
+  double s[16];
+  int c[16];
+#pragma unroll
+  for (int g = 0; g < 16; ++g) { s[g] = 0.0; c[g] = 0; }
+  unsigned act = 0, low = 0;
   int mn = 0x7fffffff;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    int v = ppc[i];
+  for (int i = block * blockDim.x + threadIdx.x; i < N; i += blocks * blockDim.x) {
+    const unsigned m = gridmask[i];
+    const int v = ppc[i];
+    float t = 0.0f;
+    if (Tnext && isBound[i]) T[i] = t = Tnext[i];
+    else if (m) t = T[i];
+    if (m) {
+#pragma unroll
+      for (int g = 0; g < 16; ++g)
+        if (g < ngrids && (m >> g & 1u)) { s[g] += (double)t; ++c[g]; }
+    }
     accum[i] += (double)v;
     if (v > 0) { ++act; if (v < 3) ++low; mn = v < mn ? v : mn; }
   }
-  const auto add = [](unsigned long long a, unsigned long long b) { return a + b; };
-  act = block_reduce(act, add, 0ull);
-  low = block_reduce(low, add, 0ull);
+  // one pair of atomics per block and grid (per-warp atomics on the same 2 * ngrids words
+  // serialised at L2)
+  const auto addd = [](double a, double b) { return a + b; };
+  const auto addu = [](unsigned a, unsigned b) { return a + b; };
+#pragma unroll
+  for (int g = 0; g < 16; ++g) {
+    if (g >= ngrids) break;
+    if (!__syncthreads_or(c[g])) continue;
+    const double a = block_reduce(s[g], addd, 0.0);
+    const unsigned b = block_reduce((unsigned)c[g], addu, 0u);
+    if (threadIdx.x == 0) { atomicAdd(sums + 2 * g, a); atomicAdd(sums + 2 * g + 1, (double)b); }
+  }
+  act = block_reduce(act, addu, 0u);
+  low = block_reduce(low, addu, 0u);
   mn = block_reduce(mn, [](int a, int b) { return a < b ? a : b; }, 0x7fffffff);
   if (threadIdx.x == 0) {
-    if (act) atomicAdd(stats, act);
-    if (low) atomicAdd(stats + 1, low);
+    if (act) atomicAdd(stats, (unsigned long long)act);
+    if (low) atomicAdd(stats + 1, (unsigned long long)low);
     atomicMin(stats + 2, (unsigned long long)mn);
   }
 }

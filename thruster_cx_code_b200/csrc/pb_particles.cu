@@ -8,7 +8,8 @@
 //  * k_count_cells       NGP cell counts clip(rint(x/dx), 1, n-2), warp-aggregated.
 //  * k_rho_finalize      rho from counts: the exact float32 result of the reference's
 //                        sequential np.add.at (ions, then electrons).
-//  * k_substep_reduce    max predicted displacement of compute_particle_substeps (:928-966).
+//  * k_substep_reduce,   max predicted displacement of compute_particle_substeps (:928-966), one
+//    k_substep_both      species (module call) or both of a step.
 //  * k_segment_hits      8-sample path absorption test (_segment_hits_grid, :1880-1901).
 //  * k_ion_step          the fused ion timestep: n_sub pushes, periodic wrap, final-cell and
 //                        path hits, impact heating, SEE spawn records, sputter damage, exit
@@ -787,14 +788,13 @@ __device__ __forceinline__ double predicted_ds(float x, float y, float vx, float
 // outside [0, nx - 2) x [0, ny - 2) cells, NaN and infinite values are never skipped.  The
 // warp shares its running maximum after each pass that evaluated any particle, so after
 // the first pass nearly every particle is skipped and the loop streams 20 B per particle.
-__global__ void __launch_bounds__(256, 4) k_substep_reduce(const float* __restrict__ x, const float* __restrict__ y,
-                                 const float* __restrict__ vx, const float* __restrict__ vy,
-                                 const float* __restrict__ vz, const int* n_dev, int n_host, const float* Ex,
-                                 const float* Ey, const float4* Ec, int nx, int ny, float dxf, float dyf, double qm,
-                                 float dtf, double dt2, unsigned long long* ds_max_bits,
-                                 const unsigned* ebound = nullptr) {
-  pdl_enter();
-  int n = n_dev ? *n_dev : n_host;
+// Block `block` of `blocks` of one species' reduction.
+__device__ __forceinline__ void substep_block(const float* __restrict__ x, const float* __restrict__ y,
+                                              const float* __restrict__ vx, const float* __restrict__ vy,
+                                              const float* __restrict__ vz, int n, const float* Ex, const float* Ey,
+                                              const float4* Ec, int nx, int ny, float dxf, float dyf, double qm,
+                                              float dtf, double dt2, unsigned long long* ds_max_bits,
+                                              const unsigned* ebound, int block, int blocks) {
   unsigned long long m = 0ull;
   const float inv_dx = __frcp_rn(dxf), inv_dy = __frcp_rn(dyf);
   // four particles per thread and pass (16-byte loads of each array), so that a thread
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(256, 4) k_substep_reduce(const float* __restri
                      reinterpret_cast<uintptr_t>(vx) | reinterpret_cast<uintptr_t>(vy) |
                      reinterpret_cast<uintptr_t>(vz)) & 15u) == 0;
   const int n4 = vec ? n >> 2 : 0;
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const int t0 = block * blockDim.x + threadIdx.x, stride = blocks * blockDim.x;
   if (vec && Ec && ebound) {
     const double acc = 0.5 * fabs(qm) * (double)__uint_as_float(__ldg(ebound)) * dt2;  // NaN, inf: no skips
     const double invdt2 = 1.0 / ((double)dtf * (double)dtf);
@@ -889,10 +889,23 @@ __global__ void __launch_bounds__(256, 4) k_substep_reduce(const float* __restri
   }
 }
 
-// n_sub for the host-facing report: read ds_max, write n_sub
-__global__ void k_substep_finish(const double* ds_max, double ds_lim, int* n_sub_out, uint32_t* errflags) {
+__global__ void __launch_bounds__(256, 4) k_substep_reduce(const float* x, const float* y, const float* vx,
+                                                           const float* vy, const float* vz, int n, const float* Ex,
+                                                           const float* Ey, const float4* Ec, int nx, int ny, float dxf,
+                                                           float dyf, double qm, float dtf, double dt2,
+                                                           unsigned long long* ds_max_bits, const unsigned* ebound) {
+  substep_block(x, y, vx, vy, vz, n, Ex, Ey, Ec, nx, ny, dxf, dyf, qm, dtf, dt2, ds_max_bits, ebound, (int)blockIdx.x,
+                (int)gridDim.x);
+}
+
+// Both species of a step in one launch: blocks below ion_blocks reduce the ions.
+__global__ void __launch_bounds__(256, 4) k_substep_both(const __grid_constant__ SubstepArgs a) {
   pdl_enter();
-  *n_sub_out = substep_count(*ds_max, ds_lim, errflags);
+  const int k = (int)blockIdx.x >= a.ion_blocks;
+  const Soa& S = a.sp[k];
+  substep_block(S.x, S.y, S.vx, S.vy, S.vz, *a.n[k], nullptr, nullptr, a.Ec, a.nx, a.ny, a.dxf, a.dyf, a.qm[k], a.dtf,
+                a.dt2, a.ds_max_bits + k, a.ebound, (int)blockIdx.x - (k ? a.ion_blocks : 0),
+                k ? (int)gridDim.x - a.ion_blocks : a.ion_blocks);
 }
 
 // ------------------------------------------------------------------ path absorption
@@ -1132,7 +1145,7 @@ __global__ void __launch_bounds__(NT, 4) k_ion_step(const __grid_constant__ IonS
   const double dt_sub = DDIV(a.dt, (double)n_sub);
   const double h = DMUL(DMUL(0.5, a.qm), dt_sub);
   const float dtf = __double2float_rn(dt_sub);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_sub_out = n_sub;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_sub_out = substep_count(*a.ds_max, a.ds_lim, a.errflags);
   const float pi_f = 3.14159265358979323846f;
   // per-thread event counts (32-bit: a thread sees far fewer than 2^32 ions); the exit
   // sums, whose ions are rare, go straight to shared memory, so neither holds registers
@@ -1417,7 +1430,7 @@ __global__ void __launch_bounds__(NT) k_ele_step(EleStepArgs a) {
   const double dt_sub = DDIV(a.dt, (double)n_sub);
   const double h = DMUL(DMUL(0.5, a.qm), dt_sub);
   const float dtf = __double2float_rn(dt_sub);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_sub_out = n_sub;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_sub_out = substep_count(*a.ds_max, a.ds_lim, a.errflags);
   while (true) {
     if (threadIdx.x == 0) sm_tile = atomicAdd(a.tile_counter, 1);
     __syncthreads();
@@ -1568,7 +1581,7 @@ __global__ void __launch_bounds__(NT, 8) k_ele_push(EleStepArgs a, uint8_t* __re
   const double dt_sub = DDIV(a.dt, (double)n_sub);
   const double h = DMUL(DMUL(0.5, a.qm), dt_sub);
   const float dtf = __double2float_rn(dt_sub);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_sub_out = n_sub;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_sub_out = substep_count(*a.ds_max, a.ds_lim, a.errflags);
   // every corner value finite (and |Ex| + |Ey| below the float range): the bound's bits
   const bool efin = a.ebound && *a.ebound < 0x7F800000u;
   // every electron's |v| finite: the sub-step reduction's maximum is finite (a NaN or

@@ -663,7 +663,9 @@ static int32_t launch_poisson(Sim* s, int iterations, const pb_step_params* p) {
 
 // The per-step resets in one launch instead of a dozen memsets (each of which is an
 // operation of its own on the GPU timeline): the step report (zero, ppc_min all ones),
-// the PPC map, both step kernels' tile descriptors and the small counters.
+// the PPC map, both step kernels' tile descriptors and the small counters.  Block 0 then
+// counts the step's injections (a launch of its own before: 8 to 14 us at a step's start, of
+// which half was waiting for the reset).
 struct StepResetArgs {
   pb_step_report* rep;
   int* ppc;
@@ -674,22 +676,28 @@ struct StepResetArgs {
   unsigned long long* ds_bits;
 };
 
-__global__ void k_step_reset(StepResetArgs a) {
+__global__ void __launch_bounds__(256) k_step_reset(const __grid_constant__ StepResetArgs a,
+                                                    const __grid_constant__ InjectArgs inject) {
   pdl_enter();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long long)gridDim.x * blockDim.x;
   static_assert(sizeof(pb_step_report) % 4 == 0 && offsetof(pb_step_report, ppc_min) % 4 == 0, "report words");
-  constexpr long long nw = sizeof(pb_step_report) / 4, w0 = offsetof(pb_step_report, ppc_min) / 4;
-  uint32_t* r = reinterpret_cast<uint32_t*>(a.rep);
-  for (long long i = tid; i < nw; i += nth) r[i] = (i == w0 || i == w0 + 1) ? 0xFFFFFFFFu : 0u;
-  for (long long i = tid; i < a.N; i += nth) a.ppc[i] = 0;
-  for (long long i = tid; i < a.ntile; i += nth) a.tile_status[i] = 0ull;
-  if (tid == 0) {
-    *a.angle_count = 0; *a.see_count = 0; *a.see_spawned = 0;
-    a.ds_bits[0] = 0ull; a.ds_bits[1] = 0ull; a.ds_bits[2] = 0ull;
-    a.tile_counter[0] = 0; a.tile_counter[1] = 0;
-    *a.ni_dst = 0; *a.ne_dst = 0;
-    for (int k = 0; k < 7; ++k) a.inj[k] = 0;
+  constexpr int nw = (int)(sizeof(pb_step_report) / 4), w0 = (int)(offsetof(pb_step_report, ppc_min) / 4);
+  if (blockIdx.x == 0) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(a.rep);
+    for (int i = threadIdx.x; i < nw; i += blockDim.x) r[i] = (i == w0 || i == w0 + 1) ? 0xFFFFFFFFu : 0u;
+    if (threadIdx.x == 0) {
+      *a.angle_count = 0; *a.see_count = 0; *a.see_spawned = 0;
+      a.ds_bits[0] = 0ull; a.ds_bits[1] = 0ull; a.ds_bits[2] = 0ull;
+      a.tile_counter[0] = 0; a.tile_counter[1] = 0;
+      *a.ni_dst = 0; *a.ne_dst = 0;
+    }
+    __syncthreads();  // the counts' error flags are words of the report
+    if (threadIdx.x < 32) inject_counts(inject);
+    if (gridDim.x > 1) return;
   }
+  const long long first = gridDim.x > 1 ? tid - blockDim.x : tid, step = gridDim.x > 1 ? nth - blockDim.x : nth;
+  for (long long i = first; i < a.N; i += step) a.ppc[i] = 0;
+  for (long long i = first; i < a.ntile; i += step) a.tile_status[i] = 0ull;
 }
 
 // RF: V_fixed on grid g = Vdc + v_rf
@@ -701,37 +709,69 @@ __global__ void k_rf_update(double* Vfixed, const double* Vdc, const uint16_t* g
 
 struct SaddleIdx { int v[8]; };
 
-// The step report's device-side fields, the saddle potential (the minimum of V over up to
-// eight saddle nodes; 0 without any) and the solver statistics, in one thread.
-__global__ void k_report(pb_step_report* r, const int* counts, int ci, int ce, const int* n_sub,
-                         const unsigned long long* ds_bits, const int* inj, const int* see_spawned, const double* V,
-                         int n_saddle, SaddleIdx sidx, const double* pstats, const uint32_t* mg_status) {
-  pdl_enter();
-  *reinterpret_cast<uint32_t*>(r + 1) = *mg_status;  // past the report: one copy brings both to the host
-  r->num_p = counts[ci];
-  r->num_e = counts[2 + ce];
-  r->n_sub_ion = n_sub[0];
-  r->n_sub_e = n_sub[1];
-  r->ds_ion = __longlong_as_double((long long)ds_bits[0]);
-  r->ds_e = __longlong_as_double((long long)ds_bits[1]);
-  r->injected = inj[0];
-  r->rf_injected = inj[1];
-  r->neut_injected = inj[2];
-  r->see_spawned = *see_spawned;
-  double mp = 0.0;
-  for (int k = 0; k < n_saddle; ++k) {
-    double v = V[sidx.v[k]];
-    mp = (k == 0 || v < mp) ? v : mp;
-  }
-  r->min_pot = mp;
-  for (int k = 0; k < 4; ++k) r->poisson_stats[k] = pstats[k];
-}
+// The end of a step in one launch: block 0 takes theta95 and writes the step report's
+// device-side fields, the saddle potential (the minimum of V over up to eight saddle nodes; 0
+// without any) and the solver statistics; the other blocks take the electrode temperatures and
+// the PPC statistics in one pass over the nodes.
+struct StepEndArgs {
+  pb_step_report* r;
+  const int *counts, *n_sub, *inj, *see_spawned;
+  int ci, ce;
+  const unsigned long long* ds_bits;
+  const double *V, *pstats;
+  int n_saddle;
+  SaddleIdx sidx;
+  const uint32_t* mg_status;
+  float* angles;
+  const int* angle_count;
+  int angle_cap;
+  uint64_t* angle_scratch;
+  // nodes
+  int N, ngrids;
+  float* T;
+  const float* Tnext;  // null: no conduction in this step
+  const uint8_t* isBound;
+  const uint16_t* gridmask;
+  const int* ppc;
+  double* accum;
+};
 
-// n_sub of both species from their reduced displacements, one thread
-__global__ void k_substep_finish2(const double* ds_max, double ds_lim, int* n_sub_out, uint32_t* errflags) {
+__global__ void __launch_bounds__(STEP_END_NT) k_step_end(const __grid_constant__ StepEndArgs a) {
   pdl_enter();
-  n_sub_out[0] = substep_count(ds_max[0], ds_lim, errflags);
-  n_sub_out[1] = substep_count(ds_max[1], ds_lim, errflags);
+  if (blockIdx.x > 0) {
+    node_stats(a.T, a.Tnext, a.isBound, a.gridmask, a.ngrids, a.r->grid_sums, a.ppc, a.accum,
+               (unsigned long long*)&a.r->ppc_active, a.N, (int)blockIdx.x - 1, (int)gridDim.x - 1);
+    return;
+  }
+  pb_step_report* const r = a.r;
+  // one field per thread, so that the loads overlap
+  switch (threadIdx.x) {
+    case 0: r->num_p = a.counts[a.ci]; break;
+    case 1: r->num_e = a.counts[2 + a.ce]; break;
+    case 2: r->n_sub_ion = a.n_sub[0]; break;
+    case 3: r->n_sub_e = a.n_sub[1]; break;
+    case 4: r->ds_ion = __longlong_as_double((long long)a.ds_bits[0]); break;
+    case 5: r->ds_e = __longlong_as_double((long long)a.ds_bits[1]); break;
+    case 6: r->injected = a.inj[0]; break;
+    case 7: r->rf_injected = a.inj[1]; break;
+    case 8: r->neut_injected = a.inj[2]; break;
+    case 9: r->see_spawned = *a.see_spawned; break;
+    case 10: *reinterpret_cast<uint32_t*>(r + 1) = *a.mg_status; break;  // past the report: one copy brings both
+    case 11: case 12: case 13: case 14: r->poisson_stats[threadIdx.x - 11] = a.pstats[threadIdx.x - 11]; break;
+    case 32: {
+      double v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = k < a.n_saddle ? a.V[a.sidx.v[k]] : 0.0;
+      double mp = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < a.n_saddle) mp = (k == 0 || v[k] < mp) ? v[k] : mp;
+      r->min_pot = mp;
+      break;
+    }
+    default: break;
+  }
+  theta95(a.angles, a.angle_count, a.angle_cap, a.angle_scratch, &r->theta95);
 }
 
 }  // namespace pb
@@ -868,17 +908,7 @@ static int32_t enqueue_step_pre(pb_sim* h, const pb_step_params* p) {
   pb_step_report* rep = s->rep_dev;
   uint32_t* ef = &rep->errflags;
 
-  // per-step resets, one launch
-  {
-    StepResetArgs r{};
-    r.rep = rep; r.ppc = s->ppc; r.N = N;
-    r.tile_status = s->tile_status; r.ntile = 2 * (long long)s->tile_cap;
-    r.angle_count = s->angle_count; r.see_count = s->see_count; r.see_spawned = s->see_spawned;
-    r.ds_bits = s->ds_bits; r.tile_counter = s->tile_counter; r.ni_dst = ni_dst; r.ne_dst = ne_dst; r.inj = s->inj;
-    CK(launch_pdl(k_step_reset, grid_for(s, std::max<long>(N, 2 * (long)s->tile_cap), 256), 256, 0, st, r));
-    ++s->launches;
-  }
-
+  // the deposit counts of the particles there are, before any injection
   if (!s->counts_valid) {
     CK(cudaMemsetAsync(s->cnt_i, 0, (size_t)N * sizeof(int), st));
     CK(cudaMemsetAsync(s->cnt_e, 0, (size_t)N * sizeof(int), st));
@@ -891,16 +921,6 @@ static int32_t enqueue_step_pre(pb_sim* h, const pb_step_params* p) {
     s->counts_valid = true;
   }
 
-  // RF co-extraction: V_fixed on one grid, then recalc_poisson(2) (:984-991)
-  int32_t rc;
-  if (p->rf_grid >= 0) {
-    CK(launch_pdl(k_rf_update, grid_for(s, N, 256), 256, 0, st, s->Vfixed, s->Vdc, s->gridmask, N, p->rf_grid,
-                  p->v_rf));
-    ++s->launches;
-    if ((rc = launch_poisson(s, 2, p))) return rc;
-  }
-
-  // A. injection (:996-1099)
   InjectArgs ia{};
   ia.ion_on = p->inject_on; ia.lam = p->lam; ia.geometry = p->geometry; ia.ylo = p->ylo; ia.yhi = p->yhi;
   for (int k = 0; k < 4; ++k) ia.span[k] = (float)p->span[k];
@@ -915,8 +935,27 @@ static int32_t enqueue_step_pre(pb_sim* h, const pb_step_params* p) {
   ia.ions = I.buf[I.cur]; ia.eles = E.buf[E.cur];
   ia.cnt_i = s->cnt_i; ia.cnt_e = s->cnt_e;
   ia.nx = s->nx; ia.ny = s->ny; ia.dxf = dxf; ia.dyf = dyf; ia.errflags = ef;
-  CK(launch_pdl(k_inject_prep, 1, 32, 0, st, ia));
-  ++s->launches;
+  // per-step resets and the injections' counts, slots and ids (:996-1099), one launch
+  {
+    StepResetArgs r{};
+    r.rep = rep; r.ppc = s->ppc; r.N = N;
+    r.tile_status = s->tile_status; r.ntile = 2 * (long long)s->tile_cap;
+    r.angle_count = s->angle_count; r.see_count = s->see_count; r.see_spawned = s->see_spawned;
+    r.ds_bits = s->ds_bits; r.tile_counter = s->tile_counter; r.ni_dst = ni_dst; r.ne_dst = ne_dst; r.inj = s->inj;
+    CK(launch_pdl(k_step_reset, 1 + grid_for(s, std::max<long>(N, 2 * (long)s->tile_cap), 256), 256, 0, st, r, ia));
+    ++s->launches;
+  }
+
+  // RF co-extraction: V_fixed on one grid, then recalc_poisson(2) (:984-991)
+  int32_t rc;
+  if (p->rf_grid >= 0) {
+    CK(launch_pdl(k_rf_update, grid_for(s, N, 256), 256, 0, st, s->Vfixed, s->Vdc, s->gridmask, N, p->rf_grid,
+                  p->v_rf));
+    ++s->launches;
+    if ((rc = launch_poisson(s, 2, p))) return rc;
+  }
+
+  // A. injection: the new particles
   {
     long mx = std::max<long>({(long)(p->lam + 40.0 * std::sqrt(std::max(p->lam, 0.0)) + 100.0),
                               (long)p->neut_n, (long)p->rf_num_float + 1, 1L});
@@ -957,16 +996,20 @@ static int32_t enqueue_step_post(pb_sim* h, const pb_step_params* p) {
 
   // C. sub-step counts (:1177-1209)
   const float dtf = (float)p->dt;
-  CK(launch_pdl(k_substep_reduce, grid_for(s, I.cap / 4, 256, 4), 256, 0, st, I.buf[I.cur].x, I.buf[I.cur].y,
-                I.buf[I.cur].vx, I.buf[I.cur].vy, I.buf[I.cur].vz, ni_src, 0, s->Ex, s->Ey, s->ecorn, s->nx, s->ny, dxf,
-                dyf, p->qm_ion, dtf, p->dt2, s->ds_bits, ebound));
-  ++s->launches;
-  CK(launch_pdl(k_substep_reduce, grid_for(s, E.cap / 4, 256, 4), 256, 0, st, E.buf[E.cur].x, E.buf[E.cur].y,
-                E.buf[E.cur].vx, E.buf[E.cur].vy, E.buf[E.cur].vz, ne_src, 0, s->Ex, s->Ey, s->ecorn, s->nx, s->ny, dxf,
-                dyf, p->qm_e, dtf, p->dt2, s->ds_bits + 1, ebound));
-  ++s->launches;
-  CK(launch_pdl(k_substep_finish2, 1, 1, 0, st, (const double*)s->ds_bits, p->ds_lim, s->n_sub, ef));
-  ++s->launches;
+  {
+    SubstepArgs sa{};
+    sa.sp[0] = I.buf[I.cur]; sa.sp[1] = E.buf[E.cur];
+    sa.n[0] = ni_src; sa.n[1] = ne_src;
+    sa.qm[0] = p->qm_ion; sa.qm[1] = p->qm_e;
+    sa.Ec = s->ecorn; sa.ebound = ebound; sa.nx = s->nx; sa.ny = s->ny; sa.dxf = dxf; sa.dyf = dyf; sa.dtf = dtf;
+    sa.dt2 = p->dt2; sa.ds_max_bits = s->ds_bits;
+    // one launch for both species, the resident blocks shared by particle count
+    const long gi = grid_for(s, I.cap / 4, 256, 4), ge = grid_for(s, E.cap / 4, 256, 4), all = 4L * s->num_sms;
+    const double share = (double)I.cap / ((double)I.cap + E.cap);
+    sa.ion_blocks = (int)(gi + ge <= all ? gi : std::min(all - 1, std::max(1L, (long)(share * all + 0.5))));
+    CK(launch_pdl(k_substep_both, (unsigned)std::min(gi + ge, all), 256, 0, st, sa));
+    ++s->launches;
+  }
   mark(s);
 
   // ions: push, hits, tallies, exit diagnostics, compaction, CEX, PPC (:1211-1739)
@@ -1067,23 +1110,19 @@ static int32_t enqueue_step_post(pb_sim* h, const pb_step_params* p) {
         (float)p->Fo_y, p->sweeps));
     ++s->launches;
   }
-  if (s->ngrids > 0 || p->thermal_on) {
-    CK(launch_pdl(k_grid_sums, grid_for(s, N, 256), 256, 0, st, s->Tmap, p->thermal_on ? s->Tnext : nullptr, s->isBound,
-                  s->gridmask, N, std::min(s->ngrids, 16), rep->grid_sums));
-    ++s->launches;
-  }
   mark(s);
 
   // exit divergence, saddle potential, PPC map (:1482-1488, 1655-1676, 1741-1767)
-  CK(launch_pdl(k_theta95, 1, 1024, 0, st, s->angles, s->angle_count, s->angle_cap, s->angle_scratch, &rep->theta95));
-  ++s->launches;
-  SaddleIdx sidx{};
-  for (int k = 0; k < 8; ++k) sidx.v[k] = p->saddle_idx[k];
-  CK(launch_pdl(k_report, 1, 1, 0, st, rep, s->counts, I.cur, E.cur, s->n_sub, s->ds_bits, s->inj, s->see_spawned, s->V,
-                            std::max(0, std::min(p->n_saddle, 8)), sidx, s->pstats, s->mg_status));
-  ++s->launches;
-  CK(launch_pdl(k_ppc_stats, grid_for(s, N, 256), 256, 0, st, s->ppc, s->accum_ppc, N,
-                (unsigned long long*)&rep->ppc_active));
+  StepEndArgs ea{};
+  ea.r = rep; ea.counts = s->counts; ea.n_sub = s->n_sub; ea.inj = s->inj; ea.see_spawned = s->see_spawned;
+  ea.ci = I.cur; ea.ce = E.cur; ea.ds_bits = s->ds_bits; ea.V = s->V; ea.pstats = s->pstats;
+  ea.n_saddle = std::max(0, std::min(p->n_saddle, 8));
+  for (int k = 0; k < 8; ++k) ea.sidx.v[k] = p->saddle_idx[k];
+  ea.mg_status = s->mg_status; ea.angles = s->angles; ea.angle_count = s->angle_count; ea.angle_cap = s->angle_cap;
+  ea.angle_scratch = s->angle_scratch;
+  ea.N = N; ea.ngrids = std::min(s->ngrids, 16); ea.T = s->Tmap; ea.Tnext = p->thermal_on ? s->Tnext : nullptr;
+  ea.isBound = s->isBound; ea.gridmask = s->gridmask; ea.ppc = s->ppc; ea.accum = s->accum_ppc;
+  CK(launch_pdl(k_step_end, 1 + grid_for(s, N, STEP_END_NT, 4), STEP_END_NT, 0, st, ea));
   ++s->launches;
 
   // periodic re-sort by cell key (locality of the gathers and deposits); the permutation
@@ -1262,7 +1301,7 @@ static int32_t run_one_step(pb_sim* h, const pb_step_params* p) {
   return enqueue_step(h, p);
 }
 
-// the report and, past it, the rebuild's status (k_report)
+// the report and, past it, the rebuild's status (k_step_end)
 static int32_t finish_report(Sim* s, pb_step_report* out, uint32_t* mg_status) {
   CK(cudaMemcpyAsync(s->rep_host, s->rep_dev, sizeof(pb_step_report) + sizeof(uint32_t), cudaMemcpyDeviceToHost,
                      s->stream));
@@ -1320,7 +1359,7 @@ int32_t pb_sim_create(pb_sim** out, int32_t device) {
   CK(dalloc(&s->see_xy, 2 * (size_t)s->see_cap));
   CK(dalloc(&s->angles, (size_t)s->angle_cap));
   CK(dalloc(&s->angle_scratch, 2 * (size_t)s->angle_cap));
-  CK(dalloc(&s->rep_dev, 2));  // the report and the words past it (k_report)
+  CK(dalloc(&s->rep_dev, 2));  // the report and the words past it (k_step_end)
   CK(cudaMemset(s->rep_dev, 0, 2 * sizeof(pb_step_report)));
   CK(dalloc(&s->step_dev, 1));
   CK(cudaMemset(s->step_dev, 0, sizeof(uint32_t)));
@@ -2234,7 +2273,7 @@ int32_t pb_compute_particle_substeps(const float* x, const float* y, const float
   const int gc = (int)std::min<long long>((G + 255) / 256, 148LL * 8);
   k_e_corners<<<gc, 256, 0, st>>>(Ex, Ey, ec, ny, nx, ebound);
   int g = (int)std::min<long>((n + 255) / 256, 148L * 16);
-  k_substep_reduce<<<g, 256, 0, st>>>(x, y, vx, vy, vz, nullptr, n, Ex, Ey, ec, nx, ny, (float)dx, (float)dy, qm,
+  k_substep_reduce<<<g, 256, 0, st>>>(x, y, vx, vy, vz, n, Ex, Ey, ec, nx, ny, (float)dx, (float)dy, qm,
                                       (float)dt, dt * dt, bits, ebound);
   unsigned long long hb = 0;
   CK(cudaMemcpyAsync(&hb, bits, sizeof(hb), cudaMemcpyDeviceToHost, st));
