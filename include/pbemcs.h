@@ -271,6 +271,14 @@ int32_t pb_sim_operator_digest(pb_sim* s, uint64_t* out);
 int32_t pb_sim_set_particles(pb_sim* s, int32_t species, int32_t n, const float* x, const float* y,
                              const float* vx, const float* vy, const float* vz, const uint8_t* cex,
                              const uint32_t* id, uint32_t next_id);
+/* pb_sim_set_particles with the next id set to max(largest id + 1, min_next_id) (also
+ * returned in *next_id) and, with sort != 0 and n > 0, pb_sim_sort of that species, as one
+ * call that overlaps them with the copies (pinned arrays overlap best).  Done when it
+ * returns; the particles are set even when the sort is refused. */
+int32_t pb_sim_upload_particles(pb_sim* s, int32_t species, int32_t n, const float* x, const float* y,
+                                const float* vx, const float* vy, const float* vz, const uint8_t* cex,
+                                const uint32_t* id, int64_t min_next_id, int32_t sort, double dx, double dy,
+                                int64_t* next_id);
 /* Re-order the particles of one species (0 ions, 1 electrons, -1 both) by cell key
  * iy * nx + ix, ix = clip(rint(x / dx), 1, nx - 2), with the device radix sort the step
  * uses every sort interval (stable: equal keys keep their order).  Particle order is

@@ -83,6 +83,8 @@ PROTOTYPES = {
     "pb_sim_set_spline": (i32, [vp, i32, i32, P(f64), P(f64), f64, f64]),
     "pb_sim_set_domain": (i32, [vp, i32, i32, i32, vp, vp, vp, i32, vp, vp, vp, vp, i32]),
     "pb_sim_set_particles": (i32, [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, u32]),
+    "pb_sim_upload_particles": (i32, [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, C.c_int64, i32, f64, f64,
+                                      P(C.c_int64)]),
     "pb_sim_get_particles": (i32, [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp]),
     "pb_sim_counts": (i32, [vp, P(i32), P(i32), P(u32), P(u32)]),
     "pb_sim_reserve": (i32, [vp, i32, i32]),
@@ -145,6 +147,22 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_raw_stream = None
+
+
+def stream_of(t):
+    """Handle of torch's current stream on CUDA tensor ``t``'s device.  torch.cuda.current_stream
+    builds a Stream object first, 1.5 us of a 6 us call."""
+    global _raw_stream
+    if not t.is_cuda:
+        raise ValueError(f"expected a CUDA tensor, but got one on {t.device}")
+    if _raw_stream is None:
+        import torch
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda i: torch.cuda.current_stream(i).cuda_stream)
+    return _raw_stream(t.get_device())
 
 
 # kernel variants of the step (pb_sim_set_kernel_options)

@@ -725,6 +725,27 @@ __global__ void k_sort_gather(Soa src, Soa dst, const uint32_t* perm, const int*
   }
 }
 
+// one array through the permutation (an upload's arrays arrive one by one)
+template <class T>
+__global__ void __launch_bounds__(256) k_gather(const T* __restrict__ src, T* __restrict__ dst,
+                                                const uint32_t* __restrict__ perm, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[perm[i]];
+}
+
+// *top = max(*top, ids): one uint32 per thread and turn, 16 bytes where the array allows
+__global__ void __launch_bounds__(256) k_max_id(const uint32_t* __restrict__ id, int n, uint32_t* top) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  uint32_t m = 0u;
+  const int n4 = (reinterpret_cast<uintptr_t>(id) & 15u) == 0 ? n >> 2 : 0;
+  for (int q = t0; q < n4; q += stride) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(id) + q);
+    m = max(max(m, max(v.x, v.y)), max(v.z, v.w));
+  }
+  for (int i = 4 * n4 + t0; i < n; i += stride) m = max(m, id[i]);
+  m = __reduce_max_sync(0xFFFFFFFFu, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(top, m);
+}
+
 // copy the device count to another slot (num_dst of a sort = num_src)
 __global__ void k_copy_int(const int* a, int* b) { pdl_enter(); *b = *a; }
 

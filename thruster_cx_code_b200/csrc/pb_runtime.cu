@@ -266,6 +266,10 @@ struct Sim {
   float *pw_vals = nullptr, *pw_out = nullptr;
   size_t pw_cap_leaves = 0, pw_cap_nodes = 0, pw_cap_h = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // large uploads (pb_sim_upload_particles): their copies' stream, made at the first one
+  cudaStream_t up = nullptr;
+  cudaEvent_t ev_up = nullptr;
+  uint32_t* up_max = nullptr;
   double last_ms = 0.0;
   // optional per-phase timing: events at 7 marks per step, reused across runs
   int profiling = 0;
@@ -797,11 +801,11 @@ static Spline spline_of(const SplineStore& st) {
   return sp;
 }
 
-static int32_t sort_species(Sim* s, int k, int ncell_bits) {
+// Keys and permutation of one species; *perm is the sorted order.
+static int32_t sort_perm(Sim* s, int k, int ncell_bits, const uint32_t** perm) {
   Species& S = s->sp[k];
   cudaStream_t st = s->stream;
   int* n_src = s->counts + 2 * k + S.cur;
-  int* n_dst = s->counts + 2 * k + (1 - S.cur);
   int cap = S.cap;
   int ntiles = (cap + SORT_TILE - 1) / SORT_TILE;
   const Soa& src = S.buf[S.cur];
@@ -824,7 +828,19 @@ static int32_t sort_species(Sim* s, int k, int ncell_bits) {
     ++s->launches;
     a = 1 - a;
   }
-  CK(launch_pdl(k_sort_gather, grid_for(s, cap, 256), 256, 0, st, src, S.buf[1 - S.cur], s->sval[a], n_src));
+  *perm = s->sval[a];
+  return PB_OK;
+}
+
+static int32_t sort_species(Sim* s, int k, int ncell_bits) {
+  Species& S = s->sp[k];
+  cudaStream_t st = s->stream;
+  int* n_src = s->counts + 2 * k + S.cur;
+  int* n_dst = s->counts + 2 * k + (1 - S.cur);
+  const uint32_t* perm;
+  int32_t rc;
+  if ((rc = sort_perm(s, k, ncell_bits, &perm))) return rc;
+  CK(launch_pdl(k_sort_gather, grid_for(s, S.cap, 256), 256, 0, st, S.buf[S.cur], S.buf[1 - S.cur], perm, n_src));
   ++s->launches;
   CK(launch_pdl(k_copy_int, 1, 1, 0, st, n_src, n_dst));
   ++s->launches;
@@ -1403,6 +1419,9 @@ int32_t pb_sim_destroy(pb_sim* h) {
   dfree(s->pw_lo); dfree(s->pw_left); dfree(s->pw_right); dfree(s->pw_hoff); dfree(s->pw_vals); dfree(s->pw_out);
   if (s->rep_host) cudaFreeHost(s->rep_host);
   if (s->rep_run) cudaFreeHost(s->rep_run);
+  if (s->up) cudaStreamDestroy(s->up);
+  if (s->ev_up) cudaEventDestroy(s->ev_up);
+  dfree(s->up_max);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -1619,6 +1638,129 @@ int32_t pb_sim_set_particles(pb_sim* h, int32_t species, int32_t n, const float*
   s->host_num[species] = n;
   s->counts_valid = false;
   return PB_OK;
+}
+
+// From this many particles an upload runs as a pipeline: its copies on a stream of their own, the
+// cell keys sorted while the other arrays are on their way, each array re-ordered behind its own
+// copy (a gather by itself keeps more of its source in L2 than one of all arrays), the largest id
+// found on the device.  UPLOAD_FIGURES
+constexpr int UPLOAD_PIPE_MIN = 1 << 20;
+
+static int32_t upload_piped(Sim* s, int k, int n, const float* const* f, const uint8_t* cex, const uint32_t* id,
+                            int bits, uint32_t* top) {
+  if (!s->up) CK(cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking));
+  if (!s->ev_up) CK(cudaEventCreateWithFlags(&s->ev_up, cudaEventDisableTiming));
+  if (!s->up_max) CK(dalloc(&s->up_max, 1));
+  Species& S = s->sp[k];
+  const Soa &b = S.buf[S.cur], &d = S.buf[1 - S.cur];
+  const size_t n4 = (size_t)n * 4;
+  const int grid = grid_for(s, n, 256);
+  const uint32_t* perm = nullptr;
+  // the stream whose event the other waits for: the copies run behind earlier work on the
+  // arrays, each gather behind its array's copy (a wait takes the event's latest record)
+  auto after = [s](cudaStream_t waiting, cudaStream_t st) {
+    const cudaError_t e = cudaEventRecord(s->ev_up, st);
+    return e != cudaSuccess ? e : cudaStreamWaitEvent(waiting, s->ev_up, 0);
+  };
+  auto column = [&](auto* dst, auto* tmp, const void* src, size_t bytes) -> int32_t {
+    if (src) CK(cudaMemcpyAsync(tmp, src, bytes, cudaMemcpyHostToDevice, s->up));
+    else CK(cudaMemsetAsync(tmp, 0, bytes, s->up));
+    if (!bits) return PB_OK;
+    CK(after(s->stream, s->up));
+    k_gather<<<grid, 256, 0, s->stream>>>(tmp, dst, perm, n);
+    CK(cudaGetLastError());
+    ++s->launches;
+    return PB_OK;
+  };
+  int32_t rc;
+  CK(after(s->up, s->stream));
+  CK(cudaMemcpyAsync(b.x, f[0], n4, cudaMemcpyHostToDevice, s->up));
+  CK(cudaMemcpyAsync(b.y, f[1], n4, cudaMemcpyHostToDevice, s->up));
+  if (bits) {
+    CK(after(s->stream, s->up));
+    if ((rc = sort_perm(s, k, bits, &perm))) return rc;
+    k_gather<<<grid, 256, 0, s->stream>>>(b.x, d.x, perm, n);
+    k_gather<<<grid, 256, 0, s->stream>>>(b.y, d.y, perm, n);
+    CK(cudaGetLastError());
+    s->launches += 2;
+  }
+  if ((rc = column(d.id, b.id, id, n4))) return rc;
+  CK(cudaMemsetAsync(s->up_max, 0, sizeof(uint32_t), s->up));
+  k_max_id<<<grid_for(s, n / 4 + 1, 256), 256, 0, s->up>>>(b.id, n, s->up_max);
+  CK(cudaGetLastError());
+  if ((rc = column(d.vx, b.vx, f[2], n4))) return rc;
+  if ((rc = column(d.vy, b.vy, f[3], n4))) return rc;
+  if ((rc = column(d.vz, b.vz, f[4], n4))) return rc;
+  if (S.ion && (rc = column(d.cex, b.cex, cex, (size_t)n))) return rc;
+  CK(cudaMemcpyAsync(top, s->up_max, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->up));
+  if (bits) {
+    k_copy_int<<<1, 1, 0, s->stream>>>(s->counts + 2 * k + S.cur, s->counts + 2 * k + (1 - S.cur));
+    CK(cudaGetLastError());
+    S.cur ^= 1;
+  }
+  return PB_OK;
+}
+
+static int32_t upload_plain(Sim* s, int k, int n, const float* const* f, const uint8_t* cex, const uint32_t* id,
+                            int bits, uint32_t* top) {
+  Species& S = s->sp[k];
+  const Soa& b = S.buf[S.cur];
+  const size_t n4 = (size_t)n * 4;
+  float* const dst[5] = {b.x, b.y, b.vx, b.vy, b.vz};
+  for (int a = 0; a < 5; ++a) CK(cudaMemcpyAsync(dst[a], f[a], n4, cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemcpyAsync(b.id, id, n4, cudaMemcpyHostToDevice, s->stream));
+  if (S.ion) {
+    if (cex) CK(cudaMemcpyAsync(b.cex, cex, n, cudaMemcpyHostToDevice, s->stream));
+    else CK(cudaMemsetAsync(b.cex, 0, n, s->stream));
+  }
+  int32_t rc;
+  if (bits && (rc = sort_species(s, k, bits))) return rc;
+  uint32_t m = 0;
+  for (int i = 0; i < n; ++i) m = std::max(m, id[i]);
+  *top = m;
+  return PB_OK;
+}
+
+int32_t pb_sim_upload_particles(pb_sim* h, int32_t species, int32_t n, const float* x, const float* y, const float* vx,
+                                const float* vy, const float* vz, const uint8_t* cex, const uint32_t* id,
+                                int64_t min_next_id, int32_t sort, double dx, double dy, int64_t* next_id) {
+  Sim* s = &h->s;
+  if (species < 0 || species > 1 || n < 0 || !next_id || (n > 0 && (!x || !y || !vx || !vy || !vz || !id)))
+    return fail(PB_ERR_ARG, "pb_sim_upload_particles");
+  int32_t rc;
+  if ((rc = alloc_species(s, species, std::max(n + n / 4 + 4096, 4096), 0))) return rc;
+  Species& S = s->sp[species];
+  const bool sorted = sort && n > 0;
+  const int32_t order = !sorted ? PB_OK
+                        : !s->domain_set ? fail(PB_ERR_STATE, "pb_sim_upload_particles: no domain to sort by")
+                        : !(dx > 0.0) || !(dy > 0.0) ? fail(PB_ERR_ARG, "pb_sim_upload_particles: spacing")
+                                                     : PB_OK;
+  int bits = 0;
+  if (sorted && order == PB_OK) {
+    s->sp_dx = dx;
+    s->sp_dy = dy;
+    const long N = (long)s->ny * s->nx;
+    for (bits = 1; (1L << bits) < N;) ++bits;
+  }
+  uint32_t top = 0;
+  CK(cudaMemcpyAsync(s->counts + 2 * species + S.cur, &n, sizeof(int), cudaMemcpyHostToDevice, s->stream));
+  if (n > 0) {
+    const float* const f[5] = {x, y, vx, vy, vz};
+    rc = (n >= UPLOAD_PIPE_MIN ? upload_piped : upload_plain)(s, species, n, f, cex, id, bits, &top);
+    // the caller's arrays are read and the particles in place when this returns, and nothing
+    // reads the arrays any more if it failed
+    const cudaError_t e = s->up ? cudaStreamSynchronize(s->up) : cudaSuccess;
+    const cudaError_t e2 = cudaStreamSynchronize(s->stream);
+    if (rc) return rc;
+    CK(e);
+    CK(e2);
+  }
+  *next_id = std::max<int64_t>(n > 0 ? (int64_t)top + 1 : 0, min_next_id);
+  const uint32_t nxt32 = (uint32_t)*next_id;
+  CK(cudaMemcpy(s->next_ids + species, &nxt32, sizeof(uint32_t), cudaMemcpyHostToDevice));
+  s->host_num[species] = n;
+  s->counts_valid = false;
+  return order;
 }
 
 int32_t pb_sim_sort(pb_sim* h, int32_t species, double dx, double dy) {

@@ -64,6 +64,7 @@ _FIELDS = {"V": (0, np.float64), "Ex": (1, np.float32), "Ey": (2, np.float32), "
 _PARTICLES = {"p_x": (0, 0), "p_y": (0, 1), "p_vx": (0, 2), "p_vy": (0, 3), "p_vz": (0, 4), "p_isCEX": (0, 5),
               "p_id": (0, 6), "e_x": (1, 0), "e_y": (1, 1), "e_vx": (1, 2), "e_vy": (1, 3), "e_vz": (1, 4),
               "e_id": (1, 6)}
+_MIRRORED = frozenset(_FIELDS) | frozenset(_PARTICLES)
 
 
 def _ptr(a):
@@ -183,6 +184,9 @@ class DigitalTwinSimulator:
         raise AttributeError(name)
 
     def __setattr__(self, name, value):
+        if name not in _MIRRORED:
+            object.__setattr__(self, name, value)
+            return
         mirrors = self.__dict__.get("_mirrors")
         if mirrors is not None and name in mirrors:
             m = mirrors[name]
@@ -398,20 +402,19 @@ class DigitalTwinSimulator:
         cex = None
         if sp == 0:
             cex = np.ascontiguousarray(np.zeros(n, bool) if is_cex is None else is_cex, dtype=np.uint8)
-        nxt = int(ids.max()) + 1 if n else 0
-        if next_id is not None:
-            nxt = max(nxt, int(next_id))
-        _lib.check(self._libh.pb_sim_set_particles(self._h, sp, n, *[_ptr(a) for a in arrs], _ptr(cex), _ptr(ids),
-                                                   nxt), "set_particles")
-        if sp == 0:
-            self.num_p, self.next_ion_id = n, nxt
-        else:
-            self.num_e, self.next_e_id = n, nxt
         if sort is None:
             sort = self.sort_every > 0 and bool(self.laplacian_lu)
-        if sort and n > 0:
-            _lib.check(self._libh.pb_sim_sort(self._h, sp, float(self.dx), float(self.dy)), "sort")
-        self._invalidate()
+        nxt = C.c_int64(-1)
+        rc = self._libh.pb_sim_upload_particles(self._h, sp, n, *[_ptr(a) for a in arrs], _ptr(cex), _ptr(ids),
+                                                0 if next_id is None else max(int(next_id), 0), int(bool(sort)),
+                                                float(self.dx), float(self.dy), C.byref(nxt))
+        if nxt.value >= 0:   # the particles are in place (even if the sort was refused)
+            if sp == 0:
+                self.num_p, self.next_ion_id = n, nxt.value
+            else:
+                self.num_e, self.next_e_id = n, nxt.value
+            self._invalidate()
+        _lib.check(rc, "set_particles")
 
     # ------------------------------------------------------------------ checkpoints
     _CKPT_FIELDS = ("V", "Ex", "Ey", "Tmap", "damage_map", "isBound", "V_fixed", "eroded_depth", "accum_ppc_map")
@@ -732,13 +735,19 @@ class DigitalTwinSimulator:
     def _apply_report(self, rep, params):
         sim_mode = params.get('sim_mode', 'Both')
         grids = params.get('grids', [])
-        self.last_report = rep
-        self.num_p, self.num_e = rep.num_p, rep.num_e
-        self.max_p = max(self.max_p, self.num_p)
-        self.max_e = max(self.max_e, self.num_e)
-        self.n_sub_ion, self.n_sub_e = rep.n_sub_ion, rep.n_sub_e
-        self.next_ion_id += rep.injected
-        self.next_e_id += rep.rf_injected + rep.neut_injected + rep.see_spawned
+        # none of these names is a mirrored array, so they are set together: __setattr__ name
+        # by name is a third of this function's 15 us
+        d = self.__dict__
+        num_p, num_e, injected, entered = rep.num_p, rep.num_e, float(rep.injected), float(rep.entered)
+        n = rep.crossed
+        crossed = float(n) if rep.exited_any > 0 else 0.0
+        d.update(last_report=rep, num_p=num_p, num_e=num_e, max_p=max(self.max_p, num_p), max_e=max(self.max_e, num_e),
+                 n_sub_ion=rep.n_sub_ion, n_sub_e=rep.n_sub_e, next_ion_id=self.next_ion_id + rep.injected,
+                 next_e_id=self.next_e_id + (rep.rf_injected + rep.neut_injected + rep.see_spawned),
+                 injected_ions_step=injected, injected_ions=self.injected_ions + injected,
+                 entered_optics_step=entered, entered_optics=self.entered_optics + entered, prev_entered=entered,
+                 transmitted_ions_step=crossed, transmitted_ions=self.transmitted_ions + crossed,
+                 transmitted3_step=crossed, lost_to_grid_step=float(rep.lost_to_grid))
         if self.verbose:
             lim = 0.25 * min(self.dx, self.dy) * 1e-3
             if rep.n_sub_ion > 1:
@@ -747,33 +756,17 @@ class DigitalTwinSimulator:
             if rep.n_sub_e > 1:
                 print(f"[Warning] Electron displacement criterion violated at iter {self.iteration}: predicted "
                       f"ds_max = {rep.ds_e:.3e} m, allowed = {lim:.3e} m, required substeps = {rep.n_sub_e}")
-        self.injected_ions_step = float(rep.injected)
-        self.injected_ions += float(rep.injected)
-        self.entered_optics_step = float(rep.entered)
-        self.entered_optics += float(rep.entered)
-        self.prev_entered = self.entered_optics_step
-        self.transmitted_ions_step = 0.0
-        self.transmitted3_step = 0.0
-        if rep.exited_any > 0:
-            self.transmitted_ions_step = float(rep.crossed)
-            self.transmitted_ions += float(rep.crossed)
-            self.transmitted3_step = float(rep.crossed)
-        self.lost_to_grid_step = float(rep.lost_to_grid)
-        s = rep.exit_sums
-        n = rep.crossed
+        nan = np.nan
         if n > 0:
-            self.exit_vx_mean = s[0] / n
-            self.exit_v_mean = s[1] / n
-            self.exit_energy_mean_eV = s[2] / n
-            self.exit_vx_std = math.sqrt(max(s[7] / n - (s[0] / n) ** 2, 0.0))
-            self.exit_v_std = math.sqrt(max(s[8] / n - (s[1] / n) ** 2, 0.0))
-            self.exit_count_step = int(n)
-            self.exit_v_mean_primary = s[3] / s[4] if s[4] > 0 else np.nan
-            self.exit_v_mean_cex = s[5] / s[6] if s[6] > 0 else np.nan
+            s = rep.exit_sums[:9]
+            d.update(exit_vx_mean=s[0] / n, exit_v_mean=s[1] / n, exit_energy_mean_eV=s[2] / n,
+                     exit_vx_std=math.sqrt(max(s[7] / n - (s[0] / n) ** 2, 0.0)),
+                     exit_v_std=math.sqrt(max(s[8] / n - (s[1] / n) ** 2, 0.0)), exit_count_step=int(n),
+                     exit_v_mean_primary=s[3] / s[4] if s[4] > 0 else nan,
+                     exit_v_mean_cex=s[5] / s[6] if s[6] > 0 else nan)
         else:
-            self.exit_vx_mean = self.exit_v_mean = self.exit_vx_std = self.exit_v_std = np.nan
-            self.exit_energy_mean_eV = self.exit_v_mean_primary = self.exit_v_mean_cex = np.nan
-            self.exit_count_step = 0
+            d.update(exit_vx_mean=nan, exit_v_mean=nan, exit_vx_std=nan, exit_v_std=nan, exit_energy_mean_eV=nan,
+                     exit_v_mean_primary=nan, exit_v_mean_cex=nan, exit_count_step=0)
         current_div = float(rep.theta95) if n > 5 else np.nan
         remeshed = False
         if rep.broken > 0:
@@ -781,19 +774,19 @@ class DigitalTwinSimulator:
             remeshed = True
         min_pot = np.float64(rep.min_pot)
         if sim_mode in ('Thermal', 'Both'):
-            for i, mask in enumerate(self.mask_grids[:16]):
-                cnt = rep.grid_sums[2 * i + 1]
-                if cnt > 0:
-                    self.T_grids[i] = np.float32(rep.grid_sums[2 * i] / cnt)
+            n_grids = min(len(self.mask_grids), 16)
+            sums = rep.grid_sums[:2 * n_grids]
+            for i in range(n_grids):
+                if sums[2 * i + 1] > 0:
+                    self.T_grids[i] = np.float32(sums[2 * i] / sums[2 * i + 1])
             if self._thermal_bow(params, grids):
                 self.build_domain(params, preserve_state=True)
                 remeshed = True
                 V = self.V
                 min_pot = min(V.ravel()[i] for i in self._saddle_indices(grids))
         trans_last_frame = self.transmitted3_step / self.entered_optics_step if self.entered_optics_step > 0 else 0.0
-        self.total_active_cells = int(rep.ppc_active)
-        self.low_ppc_cells = int(rep.ppc_low)
-        self.ppc_steps_count += 1
+        d.update(total_active_cells=int(rep.ppc_active), low_ppc_cells=int(rep.ppc_low),
+                 ppc_steps_count=self.ppc_steps_count + 1)
         if self.verbose and self.low_ppc_cells > 0:
             pct = self.low_ppc_cells / self.total_active_cells * 100.0 if self.total_active_cells else 0.0
             print(f"Warning: {self.low_ppc_cells} active cells have fewer than 3 macroparticles.")
@@ -990,16 +983,11 @@ class _GeometryState:
 
 
 # ---------------------------------------------------------------------- module-level kernels
-def _stream_of(t):
-    import torch
-    return torch.cuda.current_stream(t.device).cuda_stream
-
-
 def accumulate_rho(x, y, rho, num_p, dx, dy, nx, ny, charge_density):
     """GPU ``accumulate_rho`` (physics_engine.py:38-60, 178-185) on CUDA tensors; rho is
     updated in place with the exact float32 result of the sequential deposit."""
     _lib.check(_lib.load().pb_accumulate_rho(x.data_ptr(), y.data_ptr(), rho.data_ptr(), int(num_p), float(dx),
-                                             float(dy), int(nx), int(ny), float(charge_density), _stream_of(rho)),
+                                             float(dy), int(nx), int(ny), float(charge_density), _lib.stream_of(rho)),
                "accumulate_rho")
 
 
@@ -1008,11 +996,11 @@ def push_particles_boris(x, y, vx, vy, vz, Ex, Ey, Bx, By, Bz, num_p, dx, dy, nx
     _lib.check(_lib.load().pb_push_particles_boris(x.data_ptr(), y.data_ptr(), vx.data_ptr(), vy.data_ptr(),
                                                    vz.data_ptr(), Ex.data_ptr(), Ey.data_ptr(), Bx.data_ptr(),
                                                    By.data_ptr(), Bz.data_ptr(), int(num_p), float(dx), float(dy),
-                                                   int(nx), int(ny), float(dt), float(q_m), _stream_of(x)),
+                                                   int(nx), int(ny), float(dt), float(q_m), _lib.stream_of(x)),
                "push_particles_boris")
 
 
 def thermal_conduction(T, T_new, mask, nx, ny, Fo_x, Fo_y):
     """GPU ``thermal_conduction`` (Taichi kernel semantics, physics_engine.py:147-171)."""
     _lib.check(_lib.load().pb_thermal_conduction(T.data_ptr(), T_new.data_ptr(), mask.data_ptr(), int(nx), int(ny),
-                                                 float(Fo_x), float(Fo_y), _stream_of(T)), "thermal_conduction")
+                                                 float(Fo_x), float(Fo_y), _lib.stream_of(T)), "thermal_conduction")

@@ -32,10 +32,6 @@ def _need(t, name, dtype=_F32):
         raise RuntimeError(f"pbemcs: {name} must be contiguous")
 
 
-def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
-
-
 @torch.library.custom_op("pbemcs::accumulate_rho", mutates_args=("rho",), device_types="cuda")
 def accumulate_rho(x: torch.Tensor, y: torch.Tensor, rho: torch.Tensor, num_p: int, dx: float, dy: float,
                    nx: int, ny: int, charge_density: float) -> None:
@@ -44,7 +40,7 @@ def accumulate_rho(x: torch.Tensor, y: torch.Tensor, rho: torch.Tensor, num_p: i
     if rho.numel() < nx * ny or min(x.numel(), y.numel()) < num_p:
         raise RuntimeError("pbemcs: accumulate_rho: arrays smaller than num_p / nx * ny")
     _lib.check(_lib.load().pb_accumulate_rho(x.data_ptr(), y.data_ptr(), rho.data_ptr(), int(num_p), float(dx),
-                                             float(dy), int(nx), int(ny), float(charge_density), _stream(rho)),
+                                             float(dy), int(nx), int(ny), float(charge_density), _lib.stream_of(rho)),
                "accumulate_rho")
 
 
@@ -61,7 +57,7 @@ def push_particles_boris(x: torch.Tensor, y: torch.Tensor, vx: torch.Tensor, vy:
     _lib.check(_lib.load().pb_push_particles_boris(x.data_ptr(), y.data_ptr(), vx.data_ptr(), vy.data_ptr(),
                                                    vz.data_ptr(), Ex.data_ptr(), Ey.data_ptr(), Bx.data_ptr(),
                                                    By.data_ptr(), Bz.data_ptr(), int(num_p), float(dx), float(dy),
-                                                   int(nx), int(ny), float(dt), float(q_m), _stream(x)),
+                                                   int(nx), int(ny), float(dt), float(q_m), _lib.stream_of(x)),
                "push_particles_boris")
 
 
@@ -74,7 +70,7 @@ def thermal_conduction(T: torch.Tensor, T_new: torch.Tensor, mask: torch.Tensor,
     if min(T.numel(), T_new.numel(), mask.numel()) < nx * ny:
         raise RuntimeError("pbemcs: thermal_conduction: arrays smaller than nx * ny")
     _lib.check(_lib.load().pb_thermal_conduction(T.data_ptr(), T_new.data_ptr(), mask.data_ptr(), int(nx), int(ny),
-                                                 float(Fo_x), float(Fo_y), _stream(T)), "thermal_conduction")
+                                                 float(Fo_x), float(Fo_y), _lib.stream_of(T)), "thermal_conduction")
 
 
 # tracing (torch.compile, meta tensors): the operators return nothing and only mutate
