@@ -70,6 +70,12 @@ __device__ __forceinline__ double* vb_scratch(const PoissonArgs& a) {
   return reinterpret_cast<double*>(dyn_smem + a.vb_off);
 }
 
+// the fused phases' shared memory, after the coarsest right-hand side
+__device__ __forceinline__ float* fused_smem(const PoissonArgs& a) {
+  extern __shared__ float4 dyn_smem[];
+  return reinterpret_cast<float*>(dyn_smem + a.vb_off);
+}
+
 // grid barrier of this instance's blocks (grid_sync: bounded, release/acquire)
 __device__ __forceinline__ void grid_barrier(const PoissonArgs& a) { grid_sync(a.bar, a.errflags, a.nblk, gbid(a)); }
 
@@ -546,6 +552,43 @@ __device__ void vcycle_below(const PoissonArgs& a, float* rcs, int slot, const f
   tmark(a, 8);
 }
 
+// E = -grad V and the solve's statistics
+__device__ __forceinline__ void solve_end(const PoissonArgs& a, int tid, int nth, double n_outer, double n_inner,
+                                          double last_rel, unsigned long long t_start) {
+  const int N = a.ny * a.nx;
+  // ---- E = -grad V (np.gradient: central inside, one-sided at the edges; periodic y fix)
+  if (a.compute_field) {
+    for (int i = tid; i < N; i += nth) {
+      int y = i / a.nx, x = i - y * a.nx;
+      const double* V = a.V;
+      double ex, ey;
+      if (x == 0) ex = DDIV(DSUB(-(*(V + i + 1)), -(*(V + i))), a.hx);
+      else if (x == a.nx - 1) ex = DDIV(DSUB(-(*(V + i)), -(*(V + i - 1))), a.hx);
+      else ex = DDIV(DSUB(-(*(V + i + 1)), -(*(V + i - 1))), a.two_hx);
+      if (a.periodic && y == 0) ey = DDIV(DSUB((*(V + (size_t)(a.ny - 1) * a.nx + x)), (*(V + a.nx + x))), a.two_hy_per);
+      else if (a.periodic && y == a.ny - 1) ey = DDIV(DSUB((*(V + (size_t)(a.ny - 2) * a.nx + x)), (*(V + x))), a.two_hy_per);
+      else if (y == 0) ey = DDIV(DSUB(-(*(V + i + a.nx)), -(*(V + i))), a.hy);
+      else if (y == a.ny - 1) ey = DDIV(DSUB(-(*(V + i)), -(*(V + i - a.nx))), a.hy);
+      else ey = DDIV(DSUB(-(*(V + i + a.nx)), -(*(V + i - a.nx))), a.two_hy);
+      a.Ex[i] = __double2float_rn(ex);
+      a.Ey[i] = __double2float_rn(ey);
+    }
+  }
+  tmark(a, 19);
+  if (tid == 0) {
+    a.stats[0] += n_outer;
+    a.stats[1] += n_inner;
+    a.stats[2] = last_rel;
+    a.stats[3] += (double)a.iterations;
+  }
+  if (gbid(a) == 0 && threadIdx.x == 0) {
+    unsigned long long t_end;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
+    a.solve_ns[0] += (t_end - t_start) * (unsigned long long)a.nblk;  // block-ns
+    a.solve_ns[1] += 1;
+  }
+}
+
 // ----------------------------------------------------------------- the persistent kernel
 __device__ __forceinline__ void poisson_body(const PoissonArgs& a) {
   extern __shared__ float4 dyn_smem[];
@@ -748,40 +791,743 @@ __device__ __forceinline__ void poisson_body(const PoissonArgs& a) {
     tmark(a, 18);
   }
 
-  // ---- E = -grad V (np.gradient: central inside, one-sided at the edges; periodic y fix)
-  if (a.compute_field) {
-    for (int i = tid; i < N; i += nth) {
-      int y = i / a.nx, x = i - y * a.nx;
-      const double* V = a.V;
-      double ex, ey;
-      if (x == 0) ex = DDIV(DSUB(-(*(V + i + 1)), -(*(V + i))), a.hx);
-      else if (x == a.nx - 1) ex = DDIV(DSUB(-(*(V + i)), -(*(V + i - 1))), a.hx);
-      else ex = DDIV(DSUB(-(*(V + i + 1)), -(*(V + i - 1))), a.two_hx);
-      if (a.periodic && y == 0) ey = DDIV(DSUB((*(V + (size_t)(a.ny - 1) * a.nx + x)), (*(V + a.nx + x))), a.two_hy_per);
-      else if (a.periodic && y == a.ny - 1) ey = DDIV(DSUB((*(V + (size_t)(a.ny - 2) * a.nx + x)), (*(V + x))), a.two_hy_per);
-      else if (y == 0) ey = DDIV(DSUB(-(*(V + i + a.nx)), -(*(V + i))), a.hy);
-      else if (y == a.ny - 1) ey = DDIV(DSUB(-(*(V + i)), -(*(V + i - a.nx))), a.hy);
-      else ey = DDIV(DSUB(-(*(V + i + a.nx)), -(*(V + i - a.nx))), a.two_hy);
-      a.Ex[i] = __double2float_rn(ex);
-      a.Ey[i] = __double2float_rn(ey);
+  solve_end(a, tid, nth, n_outer, n_inner, last_rel, t_start);
+}
+
+// ----------------------------------------------------------------- fewer, longer phases
+// The body of a solve whose phases are short (PoissonArgs::fused, fused_plan).  There a phase's
+// own arithmetic is nothing; it costs a grid barrier (1.4 us), a trip to L2 for every
+// dependent load and the index arithmetic before it.  So
+//   - neighbouring phases are joined, their halos computed more than once from shared memory:
+//     the residual update with the restrictions to levels 1 and 2 (four phases of
+//     poisson_body), both fine post-sweeps with (r, z) (two), the Picard update with the next
+//     right-hand side (two);
+//   - what does not change during a launch (the nodes of the patches, their smoother weights,
+//     transfer stencils, the block's rows of the coarse inverse) is laid out in shared memory
+//     at its start: after a barrier the L1 holds none of it;
+//   - a thread keeps its own nodes' z, p, q, r and e in registers, and loads that need no
+//     total are issued before it.
+// Each value is the same expression of the same operands as in poisson_body, with the same
+// roundings (written out, so that contraction cannot differ), and each sum has its order: the
+// warps of the virtual blocks are dealt to all blocks, and every block adds the 32 warp sums
+// of a virtual block, then the virtual blocks, as vb_flush and get_sums do.  So the solve has
+// the same bits on either path.
+// 65 x 284 nodes, 5 Picard iterations, 25 CG iterations: 895 -> 585 us a call (235 barriers ->
+// 125); 129 x 568 1200 -> 926, 81 x 321 640 -> 423.  Of the 18 us that a CG iteration now takes,
+// 6 are its five barriers and 2.5 the three totals.
+// part: this virtual warp's place among the 32 nvb of a value
+__device__ __forceinline__ void vw_put(const PoissonArgs& a, int slot, int which, int part, double v) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) a.wpart[(size_t)((slot & 3) * 2 + which) * 32 * a.nvb + part] = v;
+}
+
+// The totals of one value of a slot, or of both, in two parts: the loads, then the sums (other
+// loads of a phase are issued in between).
+template <int NV>
+struct VwTotal {
+  static constexpr int NB = (FUSED_NVB_MAX + PT / 32 - 1) / (PT / 32);
+  double v[NV][NB];
+  __device__ __forceinline__ VwTotal(const PoissonArgs& a, int slot) {
+    const double* part = a.wpart + (size_t)(slot & 3) * 2 * 32 * a.nvb;
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+      for (int e = 0; e < NB; ++e) {
+        const int b = ((int)threadIdx.x >> 5) + e * (PT / 32);
+        v[q][e] = b < a.nvb ? __ldcg(part + (q * a.nvb + b) * 32 + ((int)threadIdx.x & 31)) : 0.0;
+      }
+  }
+  __device__ __forceinline__ void sums(const PoissonArgs& a, double (&t)[NV]) {
+    __shared__ double vb_sum[NV][FUSED_NVB_MAX];
+    const int lane = (int)threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+      for (int e = 0; e < NB; ++e) {
+        const int b = ((int)threadIdx.x >> 5) + e * (PT / 32);
+        if (b >= a.nvb) break;
+        const double s = warp_sum(v[q][e]);
+        if (lane == 0) vb_sum[q][b] = s;
+      }
+    __syncthreads();  // the next total is at least one grid barrier away
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double s = 0.0;
+      for (int b = lane; b < a.nvb; b += 32) s += vb_sum[q][b];
+      t[q] = __shfl_sync(0xFFFFFFFFu, warp_sum(s), 0);
     }
   }
-  tmark(a, 19);
-  if (tid == 0) {
-    a.stats[0] += n_outer;
-    a.stats[1] += n_inner;
-    a.stats[2] = last_rel;
-    a.stats[3] += (double)a.iterations;
+  __device__ __forceinline__ double sum(const PoissonArgs& a) {
+    double t[1];
+    sums(a, t);
+    return t[0];
   }
-  if (gbid(a) == 0 && threadIdx.x == 0) {
-    unsigned long long t_end;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
-    a.solve_ns[0] += (t_end - t_start) * (unsigned long long)a.nblk;  // block-ns
-    a.solve_ns[1] += 1;
+};
+
+// Shared-memory layout of a block, and its sizes: one tile of level 2 with the patches of
+// levels 1 and 0 under it, the up leg's two runs of nodes with two rows and columns around
+// them, the coarser levels' nodes, rows of the coarse inverse.
+struct FusedBlock {
+  int h, w, W, np, W1, n1, hw;      // level-2 tile, patch of level 0 (row length, nodes) and level 1
+  int *dj, *l1c, *l1i, *l2i, *l2b;  // node of level 0 (-1 outside; bit 30: the tile's own), of level 1
+  float *dd, *rp, *sp, *r1, *rw;    // smoother weight, residual, s; level 1; stencils of level 2
+  int w0, w1, n0, n;                // run patches: row lengths, nodes of the first and of both
+  int *uj, *uf;                     // node; place in z1 << 9, segment << 7 and flags
+  int zw[4];                        // row length of each segment's part of z1
+  float *ud, *mt, *rt, *m2;
+  float* z1;                        // level 1's correction on the coarse patches of the runs
+  int *zn, nz;                      // their nodes (y << 16 | x)
+  float* zu;                        // and their stencils (join1)
+  float* crow;
+};
+// A level as its two legs between levels 2 and last read it: a copy in shared memory, and this
+// block's nodes (y << 16 | x, -1 past the level's last chunk) in gtid's order
+struct FusedLevel {
+  MgLevel L;
+  int* yx;
+  int share;
+};
+enum : int { UF_Y = 1, UF_X = 2, UF_M01 = 4, UF_M10 = 8, UF_W = 16, UF_E = 32, UF_RING = 64 };
+constexpr int DJ_OWN = 1 << 30;
+
+// nodes of a level that a block takes in gtid's order, rounded up to whole chunks
+__device__ __forceinline__ int level_share(const PoissonArgs& a, int l) {
+  return 32 * (((a.lev[l].ny * a.lev[l].nx + 31) / 32 + a.nblk - 1) / a.nblk);
+}
+
+__device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c1, FusedBlock& B, FusedLevel* lv) {
+  const int tid = (int)threadIdx.x, N = a.ny * a.nx, nx = a.nx, last = a.nlevels - 1;
+  const MgLevel &L1 = a.lev[1], &L2 = a.lev[2];
+  int I0 = 0, J0 = 0;
+  B.h = B.w = 0;
+  if (gbid(a) < a.dt_y * a.dt_x) {
+    const int ty = gbid(a) / a.dt_x, tx = gbid(a) - ty * a.dt_x;
+    I0 = ty * L2.ny / a.dt_y;
+    J0 = tx * L2.nx / a.dt_x;
+    B.h = (ty + 1) * L2.ny / a.dt_y - I0;
+    B.w = (tx + 1) * L2.nx / a.dt_x - J0;
+  }
+  B.hw = B.h * B.w;
+  const int H = 4 * B.h + FUSED_HALO;
+  B.W = 4 * B.w + FUSED_HALO;
+  B.W1 = 2 * B.w + 3;
+  B.np = B.hw ? H * B.W : 0;
+  B.n1 = B.hw ? (2 * B.h + 3) * B.W1 : 0;
+  const int nv = a.nvb * PT, b0 = 32 * c0, b1 = nv + 32 * c0;
+  const int l0 = max(0, min(N, 32 * c1) - b0), l1 = max(0, min(N, nv + 32 * c1) - b1);
+  B.w0 = l0 + 4;
+  B.w1 = l1 + 4;
+  B.n0 = l0 ? 5 * B.w0 : 0;
+  B.n = B.n0 + (l1 ? 5 * B.w1 : 0);
+  float* f = fused_smem(a);
+  auto take = [&](int n) { float* const q = f; f += n; return q; };
+  auto takei = [&](int n) { return reinterpret_cast<int*>(take(n)); };
+  B.dj = takei(B.np); B.dd = take(B.np); B.rp = take(B.np); B.sp = take(B.np);
+  B.l1c = takei(B.n1); B.l1i = takei(B.n1); B.r1 = take(B.n1);
+  B.l2i = takei(B.hw); B.l2b = takei(B.hw); B.rw = take(25 * B.hw);
+  B.uj = takei(B.n); B.uf = takei(B.n); B.ud = take(B.n);
+  B.mt = take(B.n); B.rt = take(B.n); B.m2 = take(B.n);
+  for (int l = a.join1 ? 2 : 1; l <= last; ++l) {
+    const int sh = level_share(a, l), Nl = a.lev[l].ny * a.lev[l].nx, lx = a.lev[l].nx;
+    int* const t = takei(sh);
+    for (int q = tid; q < sh; q += PT) {
+      const int i = ((q >> 5) * a.nblk + gbid(a)) * 32 + (q & 31), y = i / lx;
+      t[q] = i < Nl ? (y << 16) | (i - y * lx) : -1;
+    }
+    if (tid == 0) {
+      lv[l].L = a.lev[l];
+      lv[l].yx = t;
+      lv[l].share = sh;
+    }
+  }
+  if (tid == 0) lv[1].L = a.lev[1];
+  // Level 1 under the runs: a run is one or two row segments (it may cross a row's end, and is no
+  // longer than a row); the patch of a segment is the coarse nodes that its two rows and columns
+  // on every side interpolate from.  seg: first run column, fine row, coarse origin, size, place
+  int seg_u[4], seg_c0[4], seg_w[4], seg_at[4], nz = 0;
+  B.zn = reinterpret_cast<int*>(f);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int o = q >> 1, l = o ? l1 : l0, b = o ? b1 : b0;
+    const int y = b / nx + (q & 1), x0 = b - (b / nx) * nx, first = nx - x0;  // columns of the run in its first row
+    const int ua = q & 1 ? first : 0, ub = q & 1 ? l : min(l, first);
+    seg_u[q] = ua;
+    seg_at[q] = nz;
+    seg_c0[q] = seg_w[q] = 0;
+    if (ub <= ua) continue;
+    const int xa = max(0, (q & 1 ? 0 : x0) - 2), xb = min(nx - 1, (q & 1 ? 0 : x0) + (ub - ua) - 1 + 2);
+    const int Ya = max(0, y - 2) >> 1, Yb = min(L1.ny - 1, (min(a.ny - 1, y + 2) >> 1) + 1);
+    const int Xa = xa >> 1, Xb = min(L1.nx - 1, (xb >> 1) + 1);
+    const int sw = Xb - Xa + 1, cnt = (Yb - Ya + 1) * sw;
+    seg_c0[q] = Ya << 16 | Xa;
+    seg_w[q] = sw;
+    for (int k = tid; k < cnt; k += PT) B.zn[nz + k] = (Ya + k / sw) << 16 | (Xa + k % sw);
+    nz += cnt;
+  }
+  B.nz = nz;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) B.zw[q] = seg_w[q];
+  takei(nz);
+  B.z1 = take(nz);
+  B.zu = take(a.join1 ? 18 * nz : 0);
+  B.crow = f;
+  if (a.join1) {
+    __syncthreads();
+    for (int k = tid; k < nz; k += PT) {
+      const int i = (B.zn[k] >> 16) * L1.nx + (B.zn[k] & 0xFFFF);
+#pragma unroll 6
+      for (int e = 0; e < 18; ++e) B.zu[e * nz + k] = __ldg(L1.U + (size_t)e * (L1.ny * L1.nx) + i);
+    }
+  }
+  // level-0 patch of the tile: node (4 I0 - 7, 4 J0 - 7) first
+  for (int k = tid; k < B.np; k += PT) {
+    const int ly = k / B.W, lx = k - ly * B.W, y = 4 * I0 - 7 + ly, x = 4 * J0 - 7 + lx;
+    const bool in = (unsigned)y < (unsigned)a.ny && (unsigned)x < (unsigned)nx;
+    const bool own = in && ly >= 7 && ly < 7 + 4 * B.h && lx >= 7 && lx < 7 + 4 * B.w;
+    B.dj[k] = in ? (y * nx + x) | (own ? DJ_OWN : 0) : -1;
+    B.dd[k] = in ? __ldg(a.lev[0].dinv + y * nx + x) : 0.0f;
+  }
+  // level-1 patch: node (2 I0 - 2, 2 J0 - 2) first; its place in the level-0 patch
+  for (int k = tid; k < B.n1; k += PT) {
+    const int ly = k / B.W1, lx = k - ly * B.W1, I = 2 * I0 - 2 + ly, J = 2 * J0 - 2 + lx;
+    const bool in = (unsigned)I < (unsigned)L1.ny && (unsigned)J < (unsigned)L1.nx;
+    const bool act = in && __ldg(L1.dinv + I * L1.nx + J) > 0.0f;
+    const bool own = in && ly >= 2 && ly < 2 + 2 * B.h && lx >= 2 && lx < 2 + 2 * B.w;
+    B.l1c[k] = act ? (2 * ly + 3) * B.W + 2 * lx + 3 : -1;
+    B.l1i[k] = own ? I * L1.nx + J : -1;
+  }
+  for (int k = tid; k < B.hw; k += PT) {
+    const int ly = k / B.w, lx = k - ly * B.w, ic = (I0 + ly) * L2.nx + J0 + lx;
+    B.l2i[k] = ic;
+    B.l2b[k] = 2 * ly * B.W1 + 2 * lx;
+#pragma unroll 5
+    for (int e = 0; e < 25; ++e) B.rw[e * B.hw + k] = __ldg(L2.R + (size_t)e * (L2.ny * L2.nx) + ic);
+  }
+  for (int k = tid; k < B.n; k += PT) {
+    const bool o = k >= B.n0;
+    const int q = o ? k - B.n0 : k, w = o ? B.w1 : B.w0, ly = q / w, lx = q - ly * w;
+    const int j = (o ? b1 : b0) + (ly - 2) * nx + lx - 2;
+    int uj = -1, uf = 0;
+    float d = 0.0f;
+    // a column before the first segment's row or after the second's lies in another row, and
+    // nothing reads it
+    const int g = 2 * o + (lx - 2 >= seg_u[2 * o + 1] && seg_w[2 * o + 1] > 0);
+    const int x0 = (o ? b1 : b0) - ((o ? b1 : b0) / nx) * nx, xx = g & 1 ? lx - 2 - seg_u[g] : x0 + lx - 2;
+    if (j >= 0 && j < N && xx >= 0 && xx < nx) {
+      const int y = j / nx, x = j - y * nx, Y = y >> 1, X = x >> 1;
+      uj = j;
+      d = __ldg(a.lev[0].dinv + j);
+      uf = (seg_at[g] + (Y - (seg_c0[g] >> 16)) * seg_w[g] + X - (seg_c0[g] & 0xFFFF)) << 9 | (g << 7) | (y & 1 ? UF_Y : 0) | (x & 1 ? UF_X : 0) | ((x & 1) && X + 1 < L1.nx ? UF_M01 : 0) |
+           ((y & 1) && Y + 1 < L1.ny ? UF_M10 : 0) | (x > 0 ? UF_W : 0) | (x < nx - 1 ? UF_E : 0) |
+           (ly >= 1 && ly <= 3 && lx >= 1 && lx <= w - 2 ? UF_RING : 0);
+    }
+    B.uj[k] = uj;
+    B.uf[k] = uf;
+    B.ud[k] = d;
+  }
+  const int nc = __ldg(a.nc_dev), lane = tid & 31;
+  for (int t = tid >> 5; t < a.crows; t += PT / 32) {
+    const int k = t * a.nblk + gbid(a);
+    if (k >= nc) break;
+    for (int j = lane; j < nc; j += 32) B.crow[(size_t)t * nc + j] = __ldg(a.cinv + (size_t)k * nc + j);
   }
 }
 
+// The rest of the restriction from the residual in rp: s = r - A D r, level 1, level 2.
+__device__ __forceinline__ void down_tile(const PoissonArgs& a, const FusedBlock& B) {
+  const int tid = (int)threadIdx.x, W = B.W;
+  const float *const dp = B.dd, *const rp = B.rp;
+  float* const sp = B.sp;
+  __syncthreads();
+  // the patch's outermost ring gets no s (nothing reads it)
+  for (int i = tid + W + 1; i < B.np - W - 1; i += PT) {
+    const float d = dp[i];
+    float acc = fmaf(dp[i - 1], rp[i - 1], 0.0f);
+    acc = fmaf(dp[i + 1], rp[i + 1], acc);
+    acc = fmaf(dp[i - W], rp[i - W], acc);
+    acc = fmaf(dp[i + W], rp[i + W], acc);
+    const float s = d > 0.0f ? fmaf(W_KEEP, rp[i], acc) : 0.0f;
+    sp[i] = s;
+    const int j = B.dj[i];
+    if (j >= DJ_OWN) __stcg(a.s32 + (j - DJ_OWN), s);
+  }
+  __syncthreads();
+  for (int k = tid; k < B.n1; k += PT) {
+    const int c = B.l1c[k], ic = B.l1i[k];
+    float v = 0.0f;
+    if (c >= 0) {
+      float zp[5][5];
+#pragma unroll
+      for (int u = 0; u < 5; ++u)
+#pragma unroll
+        for (int x = 0; x < 5; ++x) {
+          if ((u == 0 || u == 4) && (x == 0 || x == 4)) { zp[u][x] = 0.0f; continue; }
+          const int i = c + (u - 2) * W + x - 2;
+          zp[u][x] = __fmul_rn(dp[i], sp[i]);
+        }
+#pragma unroll
+      for (int da = -1; da <= 1; ++da)
+#pragma unroll
+        for (int db = -1; db <= 1; ++db) {
+          const int u = da + 2, x = db + 2, i = c + da * W + db;
+          const float res = fmaf(W_KEEP, sp[i], (zp[u][x - 1] + zp[u][x + 1]) + (zp[u - 1][x] + zp[u + 1][x]));
+          const float w = (da ? 0.5f : 1.0f) * (db ? 0.5f : 1.0f);
+          v = __fadd_rn(v, dp[i] > 0.0f ? __fmul_rn(w, res) : 0.0f);
+        }
+    }
+    B.r1[k] = v;
+    if (ic >= 0) __stcg(a.lev[1].r + ic, v);
+  }
+  __syncthreads();
+  for (int k = tid; k < B.hw; k += PT) {
+    const float* const rc = B.r1 + B.l2b[k];
+    float v = 0.0f;  // nodes outside level 1 are zero in r1
+#pragma unroll
+    for (int u = 0; u < 5; ++u)
+#pragma unroll
+      for (int x = 0; x < 5; ++x) v = __fadd_rn(v, __fmul_rn(B.rw[(u * 5 + x) * B.hw + k], rc[u * B.W1 + x]));
+    __stcg(a.lev[2].r + B.l2i[k], v);
+  }
+}
+
+// restrict_pre and smooth_up_pre where the grid is not periodic: entries outside the grid have
+// weight zero, so their values are read at the nearest node instead of being masked (a third
+// of the instructions).  w, stride: the node's stencil.
+__device__ __forceinline__ float restrict_leg(const MgLevel& F, const float* r, int I, int J, const float* w,
+                                              size_t stride) {
+  const int ny = F.ny, nx = F.nx, x0 = 2 * J;
+  int xo[5];
+#pragma unroll
+  for (int u = 0; u < 5; ++u) xo[u] = min(max(x0 + u - 2, 0), nx - 1);
+  float v[25];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) {
+    const float* const row = r + min(max(2 * I + t - 2, 0), ny - 1) * nx;
+#pragma unroll
+    for (int u = 0; u < 5; ++u) v[t * 5 + u] = __fmul_rn(*(w + (t * 5 + u) * stride), *(row + xo[u]));
+  }
+  float s = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 25; ++k) s = __fadd_rn(s, v[k]);
+  return s;
+}
+
+__device__ __forceinline__ float smooth_leg(const MgLevel& F, const MgLevel& C, const float* r, const float* zc, int y,
+                                            int x, const float* w, size_t stride) {
+  const int fy = F.ny, fx = F.nx, cy = C.ny, cx = C.nx, Y = y >> 1, X = x >> 1;
+  const int xm = max(x - 1, 0), xp = min(x + 1, fx - 1), Xm = max(X - 1, 0), Xp = min(X + 1, cx - 1);
+  float v[18];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const float* const row = r + min(max(y + t - 1, 0), fy - 1) * fx;
+    const float* const crow = zc + min(max(Y + t - 1, 0), cy - 1) * cx;
+    const float* const q = w + t * 3 * stride;
+    v[6 * t] = __fmul_rn(*q, *(row + xm));
+    v[6 * t + 1] = __fmul_rn(*(q + 9 * stride), *(crow + Xm));
+    v[6 * t + 2] = __fmul_rn(*(q + stride), *(row + x));
+    v[6 * t + 3] = __fmul_rn(*(q + 10 * stride), *(crow + X));
+    v[6 * t + 4] = __fmul_rn(*(q + 2 * stride), *(row + xp));
+    v[6 * t + 5] = __fmul_rn(*(q + 11 * stride), *(crow + Xp));
+  }
+  float s = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 18; ++k) s = __fadd_rn(s, v[k]);
+  return s;
+}
+
+// Level 1's correction on the coarse patches (join1; one barrier and 0.5 us less an iteration
+// on 65 x 284 and 129 x 568, past FUSED_JOIN nodes its stencils leave no room for the coarse
+// rows), then both post-sweeps of the fine level on this block's runs: m two rows and columns beyond them,
+// the first sweep one beyond, the second on this thread's own nodes (z, the residual's r).
+constexpr int UP_PRE = 2;  // nodes of the runs' patches whose r and s a thread loads ahead
+__device__ __forceinline__ void up_runs(const PoissonArgs& a, const FusedBlock& B, const FusedLevel* lv,
+                                        const bool (&in)[2], int u, float (&zo)[2], float (&ro)[2]) {
+  const int tid = (int)threadIdx.x;
+  const MgLevel &L1 = lv[1].L, &L2 = lv[2].L;
+  // r and s first: their loads run beside those of z1
+  float r0[UP_PRE], s0[UP_PRE];
+#pragma unroll
+  for (int e = 0; e < UP_PRE; ++e) {
+    const int k = tid + e * PT, j = k < B.n ? B.uj[k] : -1;
+    r0[e] = j >= 0 ? *(a.r32 + j) : 0.0f;
+    s0[e] = j >= 0 ? *(a.s32 + j) : 0.0f;
+  }
+  for (int k = tid; k < B.nz; k += PT) {
+    const int y = B.zn[k] >> 16, x = B.zn[k] & 0xFFFF;
+    B.z1[k] = a.join1 ? smooth_leg(L1, L2, L1.r, L2.z, y, x, B.zu + k, B.nz)
+                      : *(L1.z + y * L1.nx + x);
+  }
+  __syncthreads();
+  for (int k = tid, e = 0; k < B.n; k += PT, ++e) {
+    const int j = B.uj[k], f = B.uf[k];
+    float m = 0.0f, rj = 0.0f;
+    if (j >= 0) {
+      const bool m01 = f & UF_M01, m10 = f & UF_M10;
+      const float* const z = B.z1 + (f >> 9);
+      const int Lx = (f >> 7 & 3) == 0 ? B.zw[0] : (f >> 7 & 3) == 1 ? B.zw[1] : (f >> 7 & 3) == 2 ? B.zw[2] : B.zw[3];
+      float sj;
+      if (e == 0) { rj = r0[0]; sj = s0[0]; }
+      else if (UP_PRE > 1 && e == 1) { rj = r0[UP_PRE - 1]; sj = s0[UP_PRE - 1]; }
+      else { rj = *(a.r32 + j); sj = *(a.s32 + j); }
+      const float z00 = *z, z01 = m01 ? *(z + 1) : 0.0f, z10 = m10 ? *(z + Lx) : 0.0f,
+                  z11 = m01 && m10 ? *(z + Lx + 1) : 0.0f, d = B.ud[k];
+      const float wt = (f & UF_Y ? 0.5f : 1.0f) * (f & UF_X ? 0.5f : 1.0f);
+      const float pz = __fmul_rn(wt, __fadd_rn(__fadd_rn(__fadd_rn(z00, z01), z10), z11));
+      m = d > 0.0f ? fmaf(d, __fadd_rn(rj, sj), pz) : 0.0f;
+    }
+    B.mt[k] = m;
+    B.rt[k] = rj;
+  }
+  __syncthreads();
+  for (int k = tid; k < B.n; k += PT) {
+    const int f = B.uf[k];
+    float z = 0.0f;
+    if (f & UF_RING) {
+      const float* const m = B.mt + k;
+      const float d = B.ud[k];
+      const int pw = k >= B.n0 ? B.w1 : B.w0;
+      const float mw = f & UF_W ? m[-1] : 0.0f, me = f & UF_E ? m[1] : 0.0f;
+      const float acc = __fadd_rn(B.rt[k], __fadd_rn(__fadd_rn(mw, me), __fadd_rn(m[-pw], m[pw])));
+      z = d > 0.0f ? fmaf(d, acc, __fmul_rn(W_KEEP, m[0])) : 0.0f;
+    }
+    B.m2[k] = z;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int o = 0; o < 2; ++o) {
+    zo[o] = ro[o] = 0.0f;
+    if (!in[o]) continue;
+    const int pw = o ? B.w1 : B.w0, k = (o ? B.n0 : 0) + 2 * pw + u + 2, f = B.uf[k];
+    const float* const m = B.m2 + k;
+    const float d = B.ud[k];
+    ro[o] = B.rt[k];
+    float sm = 0.0f;
+    sm = __fadd_rn(sm, f & UF_W ? m[-1] : 0.0f);
+    sm = __fadd_rn(sm, f & UF_E ? m[1] : 0.0f);
+    sm = __fadd_rn(sm, m[-pw]);
+    sm = __fadd_rn(sm, m[pw]);
+    zo[o] = d > 0.0f ? fmaf(W_KEEP, m[0], __fmul_rn(d, __fadd_rn(ro[o], sm))) : 0.0f;
+  }
+}
+
+// coarse_solve with the block's rows of the inverse in shared memory; ci: the coarse nodes
+// whose right-hand side this thread gathers, zi: the node of its warp's first row
+__device__ __forceinline__ void coarse_rows(const PoissonArgs& a, const FusedBlock& B, float* rcs, int nc,
+                                            const int (&ci)[2], int zi) {
+  const float* const r = a.lev[a.nlevels - 1].r;
+  float* const z = a.lev[a.nlevels - 1].z;
+  const int tid = (int)threadIdx.x, lane = tid & 31;
+  float v[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) v[e] = ci[e] >= 0 ? *(r + ci[e]) : 0.0f;
+#pragma unroll
+  for (int e = 0; e < 2; ++e)
+    if (ci[e] >= 0) rcs[tid + e * PT] = v[e];
+  for (int k = tid + 2 * PT; k < nc; k += PT) rcs[k] = *(r + __ldg(a.cidx + k));
+  __syncthreads();
+  for (int t = tid >> 5; t * a.nblk + gbid(a) < nc; t += PT / 32) {
+    const int k = t * a.nblk + gbid(a);
+    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+    auto dot = [&](const float* row) {
+      int j = lane;
+#pragma unroll 4
+      for (; j + 96 < nc; j += 128) {
+        s0 = fmaf(row[j], rcs[j], s0);
+        s1 = fmaf(row[j + 32], rcs[j + 32], s1);
+        s2 = fmaf(row[j + 64], rcs[j + 64], s2);
+        s3 = fmaf(row[j + 96], rcs[j + 96], s3);
+      }
+      for (; j < nc; j += 32) s0 = fmaf(row[j], rcs[j], s0);
+    };
+    if (t < a.crows) dot(B.crow + (size_t)t * nc);
+    else dot(a.cinv + (size_t)k * nc);
+    float s = (s0 + s1) + (s2 + s3);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (lane == 0) __stcg(z + (t < PT / 32 ? zi : __ldg(a.cidx + k)), s);
+  }
+}
+
+// V_new of node i from the solution, then the damped Picard update
+__device__ __forceinline__ double picard_update(const PoissonArgs& a, int i) {
+  const uint8_t c = __ldg(a.cls + i);
+  double vn;
+  if (c == NC_FREE) vn = (*(a.x + i));
+  else if (c == NC_DIR) vn = __ldg(a.Vfixed + i);
+  else {
+    int y = i / a.nx, x = i - y * a.nx;
+    int sy = y, sx = x;
+    if (x == a.nx - 1) {
+      sx = x - 1;  // right: copy (y, nx-2), which may itself be a top/bottom copy
+      uint8_t cs = __ldg(a.cls + sy * a.nx + sx);
+      if (cs == NC_NEU && !a.periodic) sy = (sy == 0) ? 1 : (sy == a.ny - 1 ? a.ny - 2 : sy);
+    } else if (y == 0) sy = 1;
+    else sy = a.ny - 2;
+    int j = sy * a.nx + sx;
+    uint8_t cj = __ldg(a.cls + j);
+    vn = (cj == NC_DIR) ? __ldg(a.Vfixed + j) : (*(a.x + j));
+  }
+  if (c != NC_FREE) __stcg(a.x + i, vn);
+  const double V = DADD(DMUL(a.omega_keep, (*(a.V + i))), DMUL(a.omega_new, vn));
+  __stcg(a.V + i, V);
+  return V;
+}
+
+__device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
+  extern __shared__ float4 dyn_smem[];
+  float* rcs = reinterpret_cast<float*>(dyn_smem);
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int N = a.ny * a.nx, nx = a.nx, nv = a.nvb * PT;
+  // this block's virtual warps [c0, c1), one per warp: nodes 32 c + lane, and nv further
+  const int vw = a.nvb * 32, c0 = (int)((long long)gbid(a) * vw / a.nblk),
+            c1 = (int)((long long)(gbid(a) + 1) * vw / a.nblk), c = c0 + warp;
+  const bool act = c < c1;
+  const int part = (c % a.nvb) * 32 + c / a.nvb;
+  const int last = a.nlevels - 1;
+  int slot = 0;
+  double n_outer = 0, n_inner = 0, last_rel = 0;
+  unsigned long long t_start = 0;
+  if (gbid(a) == 0 && tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
+  tmark(a, 20);
+
+  __shared__ FusedLevel lv[MG_MAX_LEVELS];
+  FusedBlock B;
+  fused_tables(a, c0, c1, B, lv);
+  __syncthreads();
+  const int nc = __ldg(a.nc_dev);
+  int ci[2], zi = -1;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) ci[e] = tid + e * PT < nc ? __ldg(a.cidx + tid + e * PT) : -1;
+  if (warp * a.nblk + gbid(a) < nc) zi = __ldg(a.cidx + warp * a.nblk + gbid(a));
+
+  // this thread's nodes: bits 0 to 3 a free neighbour (W, E, y - 1, y + 1), 4 to 6 the diagonal,
+  // 7 a free node; the Dirichlet-neighbour sums, which only it reads
+  bool in[2];
+  int code[2];
+#pragma unroll
+  for (int o = 0; o < 2; ++o) {
+    const int i = 32 * c + lane + o * nv;
+    in[o] = act && i < N;
+    code[o] = 0;
+    if (!in[o]) continue;
+    const int y = i / nx, x = i - y * nx;
+    int j[4];
+    nbrs0(a, i, y, x, j);
+    double s = 0.0;
+    int diag = 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint8_t cl = j[k] >= 0 ? __ldg(a.cls + j[k]) : (uint8_t)NC_NEU;
+      if (cl == NC_FREE) code[o] |= 1 << k;
+      if (cl == NC_NEU) --diag;
+      if (cl == NC_DIR) s += __ldg(a.Vfixed + j[k]);
+    }
+    code[o] |= diag << 4;
+    if (__ldg(a.cls + i) == NC_FREE) {
+      code[o] |= 128;
+      a.dirsum[i] = s;
+    }
+  }
+  // (A v)_i at a free node (apply0)
+  auto apply_d = [&](int o, int i) {
+    const double *const v = a.x + i, vi = *v;
+    const double v0 = code[o] & 1 ? *(v - 1) : 0.0, v1 = code[o] & 2 ? *(v + 1) : 0.0,
+                 v2 = code[o] & 4 ? *(v - nx) : 0.0, v3 = code[o] & 8 ? *(v + nx) : 0.0;
+    return fma((double)((code[o] >> 4) & 7), vi, -DADD(DADD(DADD(DADD(0.0, v0), v1), v2), v3));
+  };
+
+  for (int pic = 0; pic < a.iterations; ++pic) {
+    const double inner_at_pic = n_inner, outer_at_pic = n_outer;
+    // the Picard update of the solve before, the right-hand side, the residual.  The update
+    // writes x off the free nodes only, which no residual reads.
+    if (act) {
+      double ff = 0.0, rr = 0.0;
+#pragma unroll 1
+      for (int o = 0; o < 2; ++o) {
+        if (!in[o]) continue;
+        const int i = 32 * c + lane + o * nv;
+        const double Vi = pic > 0 ? picard_update(a, i) : (*(a.V + i));
+        if (!(code[o] & 128)) { __stcg(a.r32 + i, 0.0f); continue; }
+        const double vm = Vi < a.V_plasma ? Vi : a.V_plasma;
+        const double rho_e = DMUL(a.qn0_neg, exp(DDIV(DSUB(vm, a.V_plasma), a.Te_up)));
+        const double rt = DADD((double)__ldg(a.rho + i), rho_e);
+        const double fi = DADD(DMUL(a.coeff, rt), a.dirsum[i]);
+        __stcg(a.f + i, fi);
+        ff = fma(fi, fi, ff);
+        const double res = DSUB(fi, apply_d(o, i));
+        __stcg(a.r32 + i, (float)res);
+        rr = fma(res, res, rr);
+      }
+      vw_put(a, slot, 0, part, ff);
+      vw_put(a, slot, 1, part, rr);
+    }
+    grid_barrier(a);
+    double norm2[2];
+    VwTotal<2>(a, slot++).sums(a, norm2);
+    const double fnorm2 = norm2[0];
+    double rnorm2 = norm2[1];
+    tmark(a, 17);
+    const double target2 = a.tol * a.tol * fnorm2;
+
+    for (int outer = 0; outer < a.max_outer && rnorm2 > target2 && fnorm2 > 0.0; ++outer) {
+      n_outer += 1;
+      double rz_old = 0.0, rr0 = rnorm2;
+      float ev[2] = {0.0f, 0.0f}, pv[2] = {0.0f, 0.0f}, qv[2] = {0.0f, 0.0f};
+      for (int k = tid; k < B.np; k += PT) {
+        const int j = B.dj[k];
+        B.rp[k] = j >= 0 ? *(a.r32 + (j & ~DJ_OWN)) : 0.0f;
+      }
+      down_tile(a, B);
+      grid_barrier(a);
+      tmark(a, 0);
+      for (int k = 0; k < a.max_inner; ++k) {
+        n_inner += 1;
+        // z = M r: the V-cycle below the fine level's restriction
+        for (int l = 2; l < last; ++l) {
+          const MgLevel &F = lv[l].L, &C = lv[l + 1].L;
+          const int* const yx = lv[l + 1].yx;
+          for (int q = tid; q < lv[l + 1].share; q += PT)
+            if (yx[q] >= 0) {
+              const int I = yx[q] >> 16, J = yx[q] & 0xFFFF, ic = I * C.nx + J;
+              __stcg(C.r + ic, restrict_leg(F, F.r, I, J, C.R + ic, (size_t)C.ny * C.nx));
+            }
+          grid_barrier(a);
+          tmark(a, l < 7 ? l : 6);
+        }
+        coarse_rows(a, B, rcs, nc, ci, zi);
+        grid_barrier(a);
+        tmark(a, 7);
+        for (int l = last - 1; l >= (a.join1 ? 2 : 1); --l) {
+          const MgLevel &F = lv[l].L, &C = lv[l + 1].L;
+          const int* const yx = lv[l].yx;
+          for (int q = tid; q < lv[l].share; q += PT)
+            if (yx[q] >= 0) {
+              const int y = yx[q] >> 16, x = yx[q] & 0xFFFF, i = y * F.nx + x;
+              __stcg(F.z + i, smooth_leg(F, C, F.r, C.z, y, x, F.U + i, (size_t)F.ny * F.nx));
+            }
+          grid_barrier(a);
+          tmark(a, 8 + (l < 7 ? l : 6));
+        }
+        float zo[2], rv[2];
+        up_runs(a, B, lv, in, 32 * warp + lane, zo, rv);
+        if (act) {
+          double rz_p = 0.0;
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            if (!in[o]) continue;
+            __stcg(a.z32 + 32 * c + lane + o * nv, zo[o]);
+            rz_p += (double)rv[o] * (double)zo[o];
+          }
+          vw_put(a, slot, 0, part, rz_p);
+        }
+        grid_barrier(a);
+        tmark(a, 8);
+        // p = z + beta p, q = A p
+        VwTotal<1> tz(a, slot++);
+        float zn[2][4];
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          const float* const z = a.z32 + 32 * c + lane + o * nv;
+          const int f = code[o];
+          zn[o][0] = f & 1 ? *(z - 1) : 0.0f;
+          zn[o][1] = f & 2 ? *(z + 1) : 0.0f;
+          zn[o][2] = f & 4 ? *(z - nx) : 0.0f;
+          zn[o][3] = f & 8 ? *(z + nx) : 0.0f;
+        }
+        const double rz = tz.sum(a);
+        const float beta = (float)(k == 0 ? 0.0 : rz / rz_old);
+        if (act) {
+          double pq_p = 0.0;
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            const bool fr = code[o] & 128;
+            const float sz = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(0.0f, zn[o][0]), zn[o][1]), zn[o][2]), zn[o][3]);
+            const float az = fmaf((float)((code[o] >> 4) & 7), zo[o], -sz);
+            pv[o] = fr ? fmaf(beta, pv[o], zo[o]) : 0.0f;
+            qv[o] = fr ? fmaf(beta, qv[o], az) : 0.0f;
+            if (in[o]) __stcg(a.q32 + 32 * c + lane + o * nv, qv[o]);
+            pq_p += (double)pv[o] * (double)qv[o];
+          }
+          vw_put(a, slot, 0, part, pq_p);
+        }
+        grid_barrier(a);
+        tmark(a, 14);
+        // e += alpha p, r -= alpha q (on the nodes and on the tile's patch), then the next
+        // V-cycle's restrictions
+        VwTotal<1> tq(a, slot++);
+        float qp[FUSED_PATCH];
+#pragma unroll
+        for (int e = 0; e < FUSED_PATCH; ++e) {
+          const int t = tid + e * PT, j = t < B.np ? B.dj[t] : -1;
+          qp[e] = j >= 0 ? *(a.q32 + (j & ~DJ_OWN)) : 0.0f;
+        }
+        const double pq = tq.sum(a);
+        const float al = (float)(pq != 0.0 ? rz / pq : 0.0);
+#pragma unroll
+        for (int e = 0; e < FUSED_PATCH; ++e) {
+          const int t = tid + e * PT;
+          if (t < B.np) B.rp[t] = fmaf(-al, qp[e], B.rp[t]);
+        }
+        if (act) {
+          double rr_p = 0.0;
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            rv[o] = fmaf(-al, qv[o], rv[o]);
+            ev[o] = fmaf(al, pv[o], ev[o]);
+            if (in[o]) __stcg(a.r32 + 32 * c + lane + o * nv, rv[o]);
+            rr_p += (double)rv[o] * (double)rv[o];
+          }
+          vw_put(a, slot, 0, part, rr_p);
+        }
+        down_tile(a, B);
+        grid_barrier(a);
+        const double rrk = VwTotal<1>(a, slot++).sum(a);
+        tmark(a, 15);
+        rz_old = rz;
+        if (rrk <= a.tol_inner * a.tol_inner * rr0 || rrk <= target2) break;  // as in poisson_body
+      }
+      // FP64 correction and true residual
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        const int i = 32 * c + lane + o * nv;
+        if (code[o] & 128) __stcg(a.x + i, (*(a.x + i)) + (double)ev[o]);
+      }
+      grid_barrier(a);
+      if (act) {
+        double rr = 0.0;
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          const int i = 32 * c + lane + o * nv;
+          if (!(code[o] & 128)) continue;
+          const double res = DSUB((*(a.f + i)), apply_d(o, i));
+          __stcg(a.r32 + i, (float)res);
+          rr = fma(res, res, rr);
+        }
+        vw_put(a, slot, 0, part, rr);
+      }
+      grid_barrier(a);
+      rnorm2 = VwTotal<1>(a, slot++).sum(a);
+      tmark(a, 16);
+    }
+    if (!(rnorm2 <= target2) && fnorm2 > 0.0 && gbid(a) == 0 && tid == 0) atomicOr(a.errflags, PB_EF_POISSON_NOCONV);
+    if (a.trace && gbid(a) == 0 && tid == 0 && pic < 5) {
+      a.trace[21 + pic] += (unsigned long long)(n_inner - inner_at_pic);
+      a.trace[26 + pic] += (unsigned long long)(n_outer - outer_at_pic);
+    }
+    last_rel = fnorm2 > 0.0 ? sqrt(rnorm2 / fnorm2) : 0.0;
+  }
+#pragma unroll 1
+  for (int o = 0; o < 2; ++o)
+    if (in[o]) picard_update(a, 32 * c + lane + o * nv);
+  grid_barrier(a);
+  tmark(a, 18);
+  solve_end(a, gtid(a), a.nblk * PT, n_outer, n_inner, last_rel, t_start);
+}
+
 __global__ void __launch_bounds__(PT, 1) k_poisson(const __grid_constant__ PoissonArgs a) { poisson_body(a); }
+__global__ void __launch_bounds__(PT, 1) k_poisson_fused(const __grid_constant__ PoissonArgs a) {
+  poisson_body_fused(a);
+}
 
 __global__ void __launch_bounds__(PT, 1) k_poisson_batch(const PoissonArgs* __restrict__ args,
                                                          const int* __restrict__ blk_map) {

@@ -201,7 +201,7 @@ struct Sim {
   uint32_t* mg_status = nullptr;
   bool erosion_seen = false;     // a step with sputter breaks was enqueued: field solves rebuild first
   long long mg_host_rebuilds = 0;
-  double* partials = nullptr;
+  double *partials = nullptr, *wpart = nullptr;
   unsigned int* bar = nullptr;
   double* pstats = nullptr;
   unsigned long long* solve_ns = nullptr;  // [block-ns, launches] of the field solves (k_poisson*)
@@ -211,6 +211,8 @@ struct Sim {
   int trace_on = 0;
   int pgrid = 0;      // blocks of the field-solve launch (<= num_sms)
   int ut_key[3] = {0, 0, 0}, ut[2] = {1, 1};  // fine up-leg tiling for (ny, nx, blocks)
+  long long fu_key[9] = {0};  // joined phases: what fused_plan was asked, and its answer
+  FusedPlan fu;
   int pbps = 8;       // step-kernel blocks per SM (the grid; tiles are handed out by a counter)
   uint32_t kopts = PB_OPT_ELE_SPLIT;  // kernel variants of the step (PB_OPT_*; the fastest measured)
   int ppb = TILE;                     // particles per block (tile) of the step kernels
@@ -576,6 +578,16 @@ static void set_up_tiles(Sim* s, PoissonArgs* a) {
   }
   a->ut_y = s->ut[0];
   a->ut_x = s->ut[1];
+  const long long key[9] = {s->ny, s->nx, a->nlevels, s->periodic, a->nu0, a->max_inner, a->nblk, a->nvb, s->ncap};
+  if (std::memcmp(key, s->fu_key, sizeof(key)) != 0) {
+    std::memcpy(s->fu_key, key, sizeof(key));
+    s->fu = fused_plan(a->lev, a->nlevels, s->periodic != 0, a->nu0, a->max_inner, a->nvb, a->nblk, s->ncap);
+  }
+  a->fused = s->fu.smem > 0;
+  a->dt_y = s->fu.ty;
+  a->dt_x = s->fu.tx;
+  a->join1 = s->fu.join1;
+  a->crows = s->fu.crows;
 }
 
 static PoissonArgs poisson_args(Sim* s, int iterations, const pb_step_params* p) {
@@ -604,7 +616,7 @@ static PoissonArgs poisson_args(Sim* s, int iterations, const pb_step_params* p)
   a.nvb = mg_virtual_blocks((long)s->ny * s->nx, s->num_sms);
   a.vb_off = mg_vb_offset(s->ncap);
   set_up_tiles(s, &a);
-  a.partials = s->partials; a.bar = s->bar;
+  a.partials = s->partials; a.wpart = s->wpart; a.bar = s->bar;
   a.errflags = &s->rep_dev->errflags;
   a.stats = s->pstats;
   a.solve_ns = s->solve_ns;
@@ -662,6 +674,7 @@ static int32_t launch_poisson(Sim* s, int iterations, const pb_step_params* p) {
   }
   PoissonArgs a = poisson_args(s, iterations, p);
   void* args[] = {&a};
+  if (a.fused) return coop_field_launch(s, (const void*)k_poisson_fused, args, 16 * (size_t)a.vb_off + s->fu.smem);
   return coop_field_launch(s, (const void*)k_poisson, args, mg_solve_smem_bytes(s->ncap, a.nvb, a.nblk));
 }
 
@@ -1196,7 +1209,7 @@ static uint64_t state_signature(const pb_sim* h) {
                         s->Ex, s->Ey, s->rho, s->Tmap, s->Tnext, s->r32, s->z32, s->p32, s->q32, s->e32, s->s32, s->m32,
                         s->ecorn,
                         s->isBound, s->cls, s->bdist, s->gridmask, s->ppc, s->cnt_i, s->cnt_e, s->cidx, s->cinv,
-                        s->partials, s->bar, s->pstats, s->ptrace, s->counts, s->next_ids, s->tile_status,
+                        s->partials, s->wpart, s->bar, s->pstats, s->ptrace, s->counts, s->next_ids, s->tile_status,
                         s->tile_counter, s->see_key, s->see_xy, s->see_count, s->angles, s->angle_scratch,
                         s->angle_count, s->ds_bits, s->n_sub, s->inj, s->see_spawned, s->skey[0], s->skey[1],
                         s->sval[0], s->sval[1], s->shist, s->sblk, s->rep_dev, h->cx.t, h->cx.c, h->see.t,
@@ -1205,6 +1218,7 @@ static uint64_t state_signature(const pb_sim* h) {
   k = fnv(k, ptrs, sizeof(ptrs));
   for (const DevLevel& L : s->lev) k = fnv_v(k, L);
   const long long vals[] = {s->ny, s->nx, s->periodic, s->ngrids, s->nc, s->trace_on, s->pgrid, s->ut[0], s->ut[1],
+                            s->fu.ty, s->fu.tx, s->fu.join1, s->fu.crows, (long long)s->fu.smem,
                             s->pbps, s->ppb, (long long)s->kopts, (long long)s->psmem, (long long)s->tile_cap, s->see_cap,
                             s->angle_cap, (long long)s->sort_cap, (long long)s->hist_cap, s->counts_valid ? 1 : 0,
                             s->max_outer, s->max_inner, s->nu, h->cx.nt, h->see.nt, s->profiling, s->ncap,
@@ -1349,8 +1363,11 @@ int32_t pb_sim_create(pb_sim** out, int32_t device) {
                           (int)mg_solve_smem_bytes(MG_MAX_COARSE, s->num_sms, 1)));
   CK(cudaFuncSetAttribute((const void*)k_poisson, cudaFuncAttributePreferredSharedMemoryCarveout,
                           (int)cudaSharedmemCarveoutMaxL1));
+  CK(cudaFuncSetAttribute((const void*)k_poisson_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)(16 * (size_t)mg_vb_offset(MG_MAX_COARSE) + FUSED_SMEM_MAX)));
   s->pgrid = s->num_sms;
   CK(dalloc(&s->partials, 4 * 2 * (size_t)s->num_sms));
+  CK(dalloc(&s->wpart, 4 * 2 * 32 * (size_t)FUSED_NVB_MAX));
   CK(dalloc(&s->bar, 2));
   CK(dalloc(&s->pstats, 4));
   CK(dalloc(&s->solve_ns, 2));
@@ -1399,7 +1416,7 @@ int32_t pb_sim_destroy(pb_sim* h) {
   if (s->step_dev) cudaFree(s->step_dev);
   if (s->ekeep) cudaFree(s->ekeep);
   free_levels(s);
-  double* d[] = {s->V, s->Vnew, s->Vfixed, s->Vdc, s->damage, s->eroded, s->accum_ppc, s->f, s->dirsum, s->partials, s->pstats};
+  double* d[] = {s->V, s->Vnew, s->Vfixed, s->Vdc, s->damage, s->eroded, s->accum_ppc, s->f, s->dirsum, s->partials, s->wpart, s->pstats};
   for (double* q : d) if (q) cudaFree(q);
   float* fl[] = {s->Ex, s->Ey, s->rho, s->Tmap, s->Tnext, s->r32, s->z32, s->p32, s->q32, s->e32, s->s32, s->m32,
                  s->see_xy, s->angles};
