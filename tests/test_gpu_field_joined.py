@@ -43,10 +43,11 @@ def _solve(PE, dx, blocks, geometry, max_coarse):
 @pytest.mark.parametrize("dx,geometry,max_coarse", [(0.025, "half_hole", 1536), (0.0311, "half_hole", 1536),
                                                     (0.019, "half_hole", 1536), (0.0125, "half_hole", 1536),
                                                     (0.01, "half_hole", 1536), (0.04, "one_hole", 1536),
-                                                    (0.025, "half_hole", 200), (0.0125, "half_hole", 300)])
+                                                    (0.025, "half_hole", 200), (0.0125, "half_hole", 300),
+                                                    (0.00625, "half_hole", 1536), (0.007, "half_hole", 300)])
 def test_joined_phases_same_bits(PE, dx, geometry, max_coarse):
     shape, ref = _solve(PE, dx, 3, geometry, max_coarse)  # fewer blocks than virtual blocks
-    for blocks in (0, 147, 61):
+    for blocks in (0, 147, 61, 18):
         got_shape, got = _solve(PE, dx, blocks, geometry, max_coarse)
         assert got_shape == shape
         for a, b in zip(ref, got):

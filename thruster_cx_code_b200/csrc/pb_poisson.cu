@@ -451,6 +451,51 @@ __device__ __forceinline__ float smooth_up_pre(const MgLevel& F, const MgLevel& 
   return s;
 }
 
+// restrict_pre and smooth_up_pre where the grid is not periodic: entries outside the grid have
+// weight zero, so their values are read at the nearest node instead of being masked (a third
+// of the instructions: 1.3 us of a leg's 3).  w, stride: the node's stencil.
+__device__ __forceinline__ float restrict_leg(const MgLevel& F, const float* r, int I, int J, const float* w,
+                                              size_t stride) {
+  const int ny = F.ny, nx = F.nx, x0 = 2 * J;
+  int xo[5];
+#pragma unroll
+  for (int u = 0; u < 5; ++u) xo[u] = min(max(x0 + u - 2, 0), nx - 1);
+  float v[25];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) {
+    const float* const row = r + min(max(2 * I + t - 2, 0), ny - 1) * nx;
+#pragma unroll
+    for (int u = 0; u < 5; ++u) v[t * 5 + u] = __fmul_rn(*(w + (t * 5 + u) * stride), *(row + xo[u]));
+  }
+  float s = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 25; ++k) s = __fadd_rn(s, v[k]);
+  return s;
+}
+
+__device__ __forceinline__ float smooth_leg(const MgLevel& F, const MgLevel& C, const float* r, const float* zc, int y,
+                                            int x, const float* w, size_t stride) {
+  const int fy = F.ny, fx = F.nx, cy = C.ny, cx = C.nx, Y = y >> 1, X = x >> 1;
+  const int xm = max(x - 1, 0), xp = min(x + 1, fx - 1), Xm = max(X - 1, 0), Xp = min(X + 1, cx - 1);
+  float v[18];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const float* const row = r + min(max(y + t - 1, 0), fy - 1) * fx;
+    const float* const crow = zc + min(max(Y + t - 1, 0), cy - 1) * cx;
+    const float* const q = w + t * 3 * stride;
+    v[6 * t] = __fmul_rn(*q, *(row + xm));
+    v[6 * t + 1] = __fmul_rn(*(q + 9 * stride), *(crow + Xm));
+    v[6 * t + 2] = __fmul_rn(*(q + stride), *(row + x));
+    v[6 * t + 3] = __fmul_rn(*(q + 10 * stride), *(crow + X));
+    v[6 * t + 4] = __fmul_rn(*(q + 2 * stride), *(row + xp));
+    v[6 * t + 5] = __fmul_rn(*(q + 11 * stride), *(crow + Xp));
+  }
+  float s = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 18; ++k) s = __fadd_rn(s, v[k]);
+  return s;
+}
+
 // grid-wide down leg: r_{l+1} from level l (all from global memory)
 template <bool LV0>
 __device__ void down_leg(const PoissonArgs& a, int level, int tid, int nth, const float* src0 = nullptr) {
@@ -464,7 +509,8 @@ __device__ void down_leg(const PoissonArgs& a, int level, int tid, int nth, cons
       const float s = restrict0(F, src0 ? src0 : F.r, I, J, C.wrapP != 0);
       __stcg(C.r + ic, __ldg(C.dinv + ic) > 0.0f ? s : 0.0f);
     } else {
-      __stcg(C.r + ic, restrict_pre(F, C, F.r, I, J, ic));
+      __stcg(C.r + ic, a.periodic ? restrict_pre(F, C, F.r, I, J, ic)
+                                  : restrict_leg(F, F.r, I, J, C.R + ic, (size_t)Nc));
     }
   }
 }
@@ -476,7 +522,8 @@ __device__ void up_leg(const PoissonArgs& a, int level, int tid, int nth) {
   const int N = F.ny * F.nx;
   for (int i = tid; i < N; i += nth) {
     const int y = i / F.nx, x = i - y * F.nx;
-    __stcg(F.z + i, smooth_up_pre(F, C, F.r, C.z, y, x, i));
+    __stcg(F.z + i, a.periodic ? smooth_up_pre(F, C, F.r, C.z, y, x, i)
+                               : smooth_leg(F, C, F.r, C.z, y, x, F.U + i, (size_t)N));
   }
 }
 
@@ -812,9 +859,15 @@ __device__ __forceinline__ void poisson_body(const PoissonArgs& a) {
 // warps of the virtual blocks are dealt to all blocks, and every block adds the 32 warp sums
 // of a virtual block, then the virtual blocks, as vb_flush and get_sums do.  So the solve has
 // the same bits on either path.
-// 65 x 284 nodes, 5 Picard iterations, 25 CG iterations: 895 -> 585 us a call (235 barriers ->
-// 125); 129 x 568 1200 -> 926, 81 x 321 640 -> 423.  Of the 18 us that a CG iteration now takes,
-// 6 are its five barriers and 2.5 the three totals.
+// A call of 5 Picard iterations, before (poisson_body) and now: 65 x 284 nodes 895 -> 582 us (235
+// barriers -> 125 in 25 CG iterations), 81 x 321 640 -> 424, 129 x 568 1200 -> 893, 257 x 1025
+// 672 -> 608, 257 x 1135 1560 -> 1347.  Of the 18 us that a CG iteration on 65 x 284 now takes, 6
+// are its four barriers and 2.5 the three totals.
+// RUNS: the fine post-sweeps run on the block's own nodes (their owners in the sums) with halos
+// of two rows, five rows of m to one of nodes, so that (r, z) is summed in the same phase; else
+// they run on the block's tile, with a barrier before the sum.  Runs win while they are short:
+// 65 x 284 582 us against 601 on tiles, 85 x 374 800 against 819; 129 x 568 (runs of 256 nodes)
+// 942 against 895.
 // part: this virtual warp's place among the 32 nvb of a value
 __device__ __forceinline__ void vw_put(const PoissonArgs& a, int slot, int which, int part, double v) {
   v = warp_sum(v);
@@ -823,9 +876,9 @@ __device__ __forceinline__ void vw_put(const PoissonArgs& a, int slot, int which
 
 // The totals of one value of a slot, or of both, in two parts: the loads, then the sums (other
 // loads of a phase are issued in between).
-template <int NV>
+template <int NV, int NVB>
 struct VwTotal {
-  static constexpr int NB = (FUSED_NVB_MAX + PT / 32 - 1) / (PT / 32);
+  static constexpr int NB = (NVB + PT / 32 - 1) / (PT / 32);
   double v[NV][NB];
   __device__ __forceinline__ VwTotal(const PoissonArgs& a, int slot) {
     const double* part = a.wpart + (size_t)(slot & 3) * 2 * 32 * a.nvb;
@@ -838,7 +891,7 @@ struct VwTotal {
       }
   }
   __device__ __forceinline__ void sums(const PoissonArgs& a, double (&t)[NV]) {
-    __shared__ double vb_sum[NV][FUSED_NVB_MAX];
+    __shared__ double vb_sum[NV][NVB];
     const int lane = (int)threadIdx.x & 31;
 #pragma unroll
     for (int q = 0; q < NV; ++q)
@@ -877,8 +930,11 @@ struct FusedBlock {
   float *ud, *mt, *rt, *m2;
   float* z1;                        // level 1's correction on the coarse patches of the runs
   int *zn, nz;                      // their nodes (y << 16 | x)
-  float* zu;                        // and their stencils (join1)
+  float* zu;                        // and their stencils
+  int *zj, n2, W2;                  // level 2 under the tile's corrections: node (-1 outside)
+  float* z2;
   float* crow;
+  int crows;
 };
 // A level as its two legs between levels 2 and last read it: a copy in shared memory, and this
 // block's nodes (y << 16 | x, -1 past the level's last chunk) in gtid's order
@@ -887,7 +943,7 @@ struct FusedLevel {
   int* yx;
   int share;
 };
-enum : int { UF_Y = 1, UF_X = 2, UF_M01 = 4, UF_M10 = 8, UF_W = 16, UF_E = 32, UF_RING = 64 };
+enum : int { UF_Y = 1, UF_X = 2, UF_M01 = 4, UF_M10 = 8, UF_W = 16, UF_E = 32, UF_RING = 64, UF_M = 128 };
 constexpr int DJ_OWN = 1 << 30;
 
 // nodes of a level that a block takes in gtid's order, rounded up to whole chunks
@@ -895,6 +951,7 @@ __device__ __forceinline__ int level_share(const PoissonArgs& a, int l) {
   return 32 * (((a.lev[l].ny * a.lev[l].nx + 31) / 32 + a.nblk - 1) / a.nblk);
 }
 
+template <bool RUNS>
 __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c1, FusedBlock& B, FusedLevel* lv) {
   const int tid = (int)threadIdx.x, N = a.ny * a.nx, nx = a.nx, last = a.nlevels - 1;
   const MgLevel &L1 = a.lev[1], &L2 = a.lev[2];
@@ -908,17 +965,18 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     B.w = (tx + 1) * L2.nx / a.dt_x - J0;
   }
   B.hw = B.h * B.w;
-  const int H = 4 * B.h + FUSED_HALO;
-  B.W = 4 * B.w + FUSED_HALO;
-  B.W1 = 2 * B.w + 3;
+  constexpr int halo = RUNS ? FUSED_HALO : FUSED_HALO_TILE, halo1 = RUNS ? 3 : 5;
+  const int H = 4 * B.h + halo;
+  B.W = 4 * B.w + halo;
+  B.W1 = 2 * B.w + halo1;
   B.np = B.hw ? H * B.W : 0;
-  B.n1 = B.hw ? (2 * B.h + 3) * B.W1 : 0;
+  B.n1 = B.hw ? (2 * B.h + halo1) * B.W1 : 0;
   const int nv = a.nvb * PT, b0 = 32 * c0, b1 = nv + 32 * c0;
   const int l0 = max(0, min(N, 32 * c1) - b0), l1 = max(0, min(N, nv + 32 * c1) - b1);
   B.w0 = l0 + 4;
   B.w1 = l1 + 4;
   B.n0 = l0 ? 5 * B.w0 : 0;
-  B.n = B.n0 + (l1 ? 5 * B.w1 : 0);
+  B.n = RUNS ? B.n0 + (l1 ? 5 * B.w1 : 0) : 0;
   float* f = fused_smem(a);
   auto take = [&](int n) { float* const q = f; f += n; return q; };
   auto takei = [&](int n) { return reinterpret_cast<int*>(take(n)); };
@@ -926,8 +984,10 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
   B.l1c = takei(B.n1); B.l1i = takei(B.n1); B.r1 = take(B.n1);
   B.l2i = takei(B.hw); B.l2b = takei(B.hw); B.rw = take(25 * B.hw);
   B.uj = takei(B.n); B.uf = takei(B.n); B.ud = take(B.n);
-  B.mt = take(B.n); B.rt = take(B.n); B.m2 = take(B.n);
-  for (int l = a.join1 ? 2 : 1; l <= last; ++l) {
+  B.mt = take(RUNS ? B.n : B.np);
+  B.rt = take(B.n);
+  B.m2 = RUNS ? take(B.n) : B.sp;  // s is not read any more when the first post-sweep is written
+  for (int l = 2; l <= last; ++l) {
     const int sh = level_share(a, l), Nl = a.lev[l].ny * a.lev[l].nx, lx = a.lev[l].nx;
     int* const t = takei(sh);
     for (int q = tid; q < sh; q += PT) {
@@ -946,8 +1006,23 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
   // on every side interpolate from.  seg: first run column, fine row, coarse origin, size, place
   int seg_u[4], seg_c0[4], seg_w[4], seg_at[4], nz = 0;
   B.zn = reinterpret_cast<int*>(f);
+  if (!RUNS && B.hw) {
+    // the coarse nodes that the tile and two rows and columns around it interpolate from, each as
+    // its places in the patches of level 1 (the right-hand side) and level 2 (the correction)
+    const int Ya = max(0, 2 * I0 - 1), Yb = min(L1.ny - 1, 2 * (I0 + B.h) + 1);
+    const int Xa = max(0, 2 * J0 - 1), Xb = min(L1.nx - 1, 2 * (J0 + B.w) + 1), sw = Xb - Xa + 1;
+    B.W2 = B.w + 4;
+    B.n2 = (B.h + 4) * B.W2;
+    nz = (Yb - Ya + 1) * sw;
+    seg_c0[0] = Ya << 16 | Xa;
+    seg_w[0] = sw;
+    for (int k = tid; k < nz; k += PT) {
+      const int y = Ya + k / sw, x = Xa + k % sw;
+      B.zn[k] = ((y - 2 * I0 + 2) * B.W1 + x - 2 * J0 + 2) << 16 | (((y >> 1) - I0 + 2) * B.W2 + (x >> 1) - J0 + 2);
+    }
+  }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < (RUNS ? 4 : 0); ++q) {
     const int o = q >> 1, l = o ? l1 : l0, b = o ? b1 : b0;
     const int y = b / nx + (q & 1), x0 = b - (b / nx) * nx, first = nx - x0;  // columns of the run in its first row
     const int ua = q & 1 ? first : 0, ub = q & 1 ? l : min(l, first);
@@ -966,18 +1041,27 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
   }
   B.nz = nz;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) B.zw[q] = seg_w[q];
+  for (int q = 0; q < 4; ++q) B.zw[q] = RUNS || q == 0 ? seg_w[q] : 0;
   takei(nz);
   B.z1 = take(nz);
-  B.zu = take(a.join1 ? 18 * nz : 0);
-  B.crow = f;
-  if (a.join1) {
-    __syncthreads();
-    for (int k = tid; k < nz; k += PT) {
-      const int i = (B.zn[k] >> 16) * L1.nx + (B.zn[k] & 0xFFFF);
-#pragma unroll 6
-      for (int e = 0; e < 18; ++e) B.zu[e * nz + k] = __ldg(L1.U + (size_t)e * (L1.ny * L1.nx) + i);
+  B.zu = take(18 * nz);
+  if (!RUNS) {
+    if (!B.hw) B.n2 = B.W2 = 0;
+    B.zj = takei(B.n2);
+    B.z2 = take(B.n2);
+    B.uf = takei(B.np);
+    for (int k = tid; k < B.n2; k += PT) {
+      const int y = I0 - 2 + k / B.W2, x = J0 - 2 + k % B.W2;
+      B.zj[k] = (unsigned)y < (unsigned)L2.ny && (unsigned)x < (unsigned)L2.nx ? y * L2.nx + x : -1;
     }
+  }
+  B.crow = f;
+  __syncthreads();
+  for (int k = tid; k < nz; k += PT) {
+    const int i = RUNS ? (B.zn[k] >> 16) * L1.nx + (B.zn[k] & 0xFFFF)
+                       : ((seg_c0[0] >> 16) + k / seg_w[0]) * L1.nx + (seg_c0[0] & 0xFFFF) + k % seg_w[0];
+#pragma unroll 6
+    for (int e = 0; e < 18; ++e) B.zu[e * nz + k] = __ldg(L1.U + (size_t)e * (L1.ny * L1.nx) + i);
   }
   // level-0 patch of the tile: node (4 I0 - 7, 4 J0 - 7) first
   for (int k = tid; k < B.np; k += PT) {
@@ -986,6 +1070,15 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     const bool own = in && ly >= 7 && ly < 7 + 4 * B.h && lx >= 7 && lx < 7 + 4 * B.w;
     B.dj[k] = in ? (y * nx + x) | (own ? DJ_OWN : 0) : -1;
     B.dd[k] = in ? __ldg(a.lev[0].dinv + y * nx + x) : 0.0f;
+    if (!RUNS) {
+      const int py = ly - 7, px = lx - 7, Y = y >> 1, X = x >> 1;  // distance from the tile
+      int uf = 0;
+      if (in && py >= -2 && py < 4 * B.h + 2 && px >= -2 && px < 4 * B.w + 2)
+        uf = ((Y - (seg_c0[0] >> 16)) * seg_w[0] + X - (seg_c0[0] & 0xFFFF)) << 9 | UF_M | (y & 1 ? UF_Y : 0) |
+             (x & 1 ? UF_X : 0) | ((x & 1) && X + 1 < L1.nx ? UF_M01 : 0) | ((y & 1) && Y + 1 < L1.ny ? UF_M10 : 0) |
+             (py >= -1 && py < 4 * B.h + 1 && px >= -1 && px < 4 * B.w + 1 ? UF_RING : 0);
+      B.uf[k] = uf;
+    }
   }
   // level-1 patch: node (2 I0 - 2, 2 J0 - 2) first; its place in the level-0 patch
   for (int k = tid; k < B.n1; k += PT) {
@@ -1026,7 +1119,8 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     B.ud[k] = d;
   }
   const int nc = __ldg(a.nc_dev), lane = tid & 31;
-  for (int t = tid >> 5; t < a.crows; t += PT / 32) {
+  B.crows = min((int)((size_t)a.croom / max(nc, 1)), (nc + a.nblk - 1) / a.nblk);
+  for (int t = tid >> 5; t < B.crows; t += PT / 32) {
     const int k = t * a.nblk + gbid(a);
     if (k >= nc) break;
     for (int j = lane; j < nc; j += 32) B.crow[(size_t)t * nc + j] = __ldg(a.cinv + (size_t)k * nc + j);
@@ -1034,6 +1128,7 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
 }
 
 // The rest of the restriction from the residual in rp: s = r - A D r, level 1, level 2.
+template <bool RUNS>
 __device__ __forceinline__ void down_tile(const PoissonArgs& a, const FusedBlock& B) {
   const int tid = (int)threadIdx.x, W = B.W;
   const float *const dp = B.dd, *const rp = B.rp;
@@ -1048,12 +1143,12 @@ __device__ __forceinline__ void down_tile(const PoissonArgs& a, const FusedBlock
     acc = fmaf(dp[i + W], rp[i + W], acc);
     const float s = d > 0.0f ? fmaf(W_KEEP, rp[i], acc) : 0.0f;
     sp[i] = s;
-    const int j = B.dj[i];
-    if (j >= DJ_OWN) __stcg(a.s32 + (j - DJ_OWN), s);
+    const int j = RUNS ? B.dj[i] : 0;
+    if (RUNS && j >= DJ_OWN) __stcg(a.s32 + (j - DJ_OWN), s);
   }
   __syncthreads();
   for (int k = tid; k < B.n1; k += PT) {
-    const int c = B.l1c[k], ic = B.l1i[k];
+    const int c = B.l1c[k], ic = RUNS ? B.l1i[k] : -1;
     float v = 0.0f;
     if (c >= 0) {
       float zp[5][5];
@@ -1076,7 +1171,7 @@ __device__ __forceinline__ void down_tile(const PoissonArgs& a, const FusedBlock
         }
     }
     B.r1[k] = v;
-    if (ic >= 0) __stcg(a.lev[1].r + ic, v);
+    if (RUNS && ic >= 0) __stcg(a.lev[1].r + ic, v);
   }
   __syncthreads();
   for (int k = tid; k < B.hw; k += PT) {
@@ -1090,58 +1185,12 @@ __device__ __forceinline__ void down_tile(const PoissonArgs& a, const FusedBlock
   }
 }
 
-// restrict_pre and smooth_up_pre where the grid is not periodic: entries outside the grid have
-// weight zero, so their values are read at the nearest node instead of being masked (a third
-// of the instructions).  w, stride: the node's stencil.
-__device__ __forceinline__ float restrict_leg(const MgLevel& F, const float* r, int I, int J, const float* w,
-                                              size_t stride) {
-  const int ny = F.ny, nx = F.nx, x0 = 2 * J;
-  int xo[5];
-#pragma unroll
-  for (int u = 0; u < 5; ++u) xo[u] = min(max(x0 + u - 2, 0), nx - 1);
-  float v[25];
-#pragma unroll
-  for (int t = 0; t < 5; ++t) {
-    const float* const row = r + min(max(2 * I + t - 2, 0), ny - 1) * nx;
-#pragma unroll
-    for (int u = 0; u < 5; ++u) v[t * 5 + u] = __fmul_rn(*(w + (t * 5 + u) * stride), *(row + xo[u]));
-  }
-  float s = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 25; ++k) s = __fadd_rn(s, v[k]);
-  return s;
-}
-
-__device__ __forceinline__ float smooth_leg(const MgLevel& F, const MgLevel& C, const float* r, const float* zc, int y,
-                                            int x, const float* w, size_t stride) {
-  const int fy = F.ny, fx = F.nx, cy = C.ny, cx = C.nx, Y = y >> 1, X = x >> 1;
-  const int xm = max(x - 1, 0), xp = min(x + 1, fx - 1), Xm = max(X - 1, 0), Xp = min(X + 1, cx - 1);
-  float v[18];
-#pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    const float* const row = r + min(max(y + t - 1, 0), fy - 1) * fx;
-    const float* const crow = zc + min(max(Y + t - 1, 0), cy - 1) * cx;
-    const float* const q = w + t * 3 * stride;
-    v[6 * t] = __fmul_rn(*q, *(row + xm));
-    v[6 * t + 1] = __fmul_rn(*(q + 9 * stride), *(crow + Xm));
-    v[6 * t + 2] = __fmul_rn(*(q + stride), *(row + x));
-    v[6 * t + 3] = __fmul_rn(*(q + 10 * stride), *(crow + X));
-    v[6 * t + 4] = __fmul_rn(*(q + 2 * stride), *(row + xp));
-    v[6 * t + 5] = __fmul_rn(*(q + 11 * stride), *(crow + Xp));
-  }
-  float s = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 18; ++k) s = __fadd_rn(s, v[k]);
-  return s;
-}
-
-// Level 1's correction on the coarse patches (join1; one barrier and 0.5 us less an iteration
-// on 65 x 284 and 129 x 568, past FUSED_JOIN nodes its stencils leave no room for the coarse
-// rows), then both post-sweeps of the fine level on this block's runs: m two rows and columns beyond them,
+// Level 1's correction on the coarse patches, then both post-sweeps of the fine level on this
+// block's runs: m two rows and columns beyond them,
 // the first sweep one beyond, the second on this thread's own nodes (z, the residual's r).
 constexpr int UP_PRE = 2;  // nodes of the runs' patches whose r and s a thread loads ahead
 __device__ __forceinline__ void up_runs(const PoissonArgs& a, const FusedBlock& B, const FusedLevel* lv,
-                                        const bool (&in)[2], int u, float (&zo)[2], float (&ro)[2]) {
+                                        const bool (&in)[2], int u, float (&zo)[2]) {
   const int tid = (int)threadIdx.x;
   const MgLevel &L1 = lv[1].L, &L2 = lv[2].L;
   // r and s first: their loads run beside those of z1
@@ -1154,8 +1203,7 @@ __device__ __forceinline__ void up_runs(const PoissonArgs& a, const FusedBlock& 
   }
   for (int k = tid; k < B.nz; k += PT) {
     const int y = B.zn[k] >> 16, x = B.zn[k] & 0xFFFF;
-    B.z1[k] = a.join1 ? smooth_leg(L1, L2, L1.r, L2.z, y, x, B.zu + k, B.nz)
-                      : *(L1.z + y * L1.nx + x);
+    B.z1[k] = smooth_leg(L1, L2, L1.r, L2.z, y, x, B.zu + k, B.nz);
   }
   __syncthreads();
   for (int k = tid, e = 0; k < B.n; k += PT, ++e) {
@@ -1195,18 +1243,76 @@ __device__ __forceinline__ void up_runs(const PoissonArgs& a, const FusedBlock& 
   __syncthreads();
 #pragma unroll
   for (int o = 0; o < 2; ++o) {
-    zo[o] = ro[o] = 0.0f;
+    zo[o] = 0.0f;
     if (!in[o]) continue;
     const int pw = o ? B.w1 : B.w0, k = (o ? B.n0 : 0) + 2 * pw + u + 2, f = B.uf[k];
     const float* const m = B.m2 + k;
     const float d = B.ud[k];
-    ro[o] = B.rt[k];
     float sm = 0.0f;
     sm = __fadd_rn(sm, f & UF_W ? m[-1] : 0.0f);
     sm = __fadd_rn(sm, f & UF_E ? m[1] : 0.0f);
     sm = __fadd_rn(sm, m[-pw]);
     sm = __fadd_rn(sm, m[pw]);
-    zo[o] = d > 0.0f ? fmaf(W_KEEP, m[0], __fmul_rn(d, __fadd_rn(ro[o], sm))) : 0.0f;
+    zo[o] = d > 0.0f ? fmaf(W_KEEP, m[0], __fmul_rn(d, __fadd_rn(B.rt[k], sm))) : 0.0f;
+  }
+}
+
+// The same on the block's tile, for grids whose runs are too long for their patches: r, s and
+// level 1's right-hand side are the restriction's own patches, so only level 2's correction is
+// read; z goes to memory for the owners of the sums.
+__device__ __forceinline__ void up_tile(const PoissonArgs& a, const FusedBlock& B) {
+  const int tid = (int)threadIdx.x, W = B.W;
+  const float* const zc = a.lev[2].z;
+  for (int k = tid; k < B.n2; k += PT) B.z2[k] = B.zj[k] >= 0 ? *(zc + B.zj[k]) : 0.0f;
+  __syncthreads();
+  for (int k = tid; k < B.nz; k += PT) {
+    const float* const r = B.r1 + (B.zn[k] >> 16) - B.W1 - 1;
+    const float* const z = B.z2 + (B.zn[k] & 0xFFFF) - B.W2 - 1;
+    const float* const w = B.zu + k;
+    float v = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        v = __fadd_rn(v, __fmul_rn(w[(t * 3 + u) * B.nz], r[t * B.W1 + u]));
+        v = __fadd_rn(v, __fmul_rn(w[(9 + t * 3 + u) * B.nz], z[t * B.W2 + u]));
+      }
+    B.z1[k] = v;
+  }
+  __syncthreads();
+  for (int k = tid; k < B.np; k += PT) {
+    const int f = B.uf[k];
+    float m = 0.0f;
+    if (f & UF_M) {
+      const bool m01 = f & UF_M01, m10 = f & UF_M10;
+      const float* const z = B.z1 + (f >> 9);
+      const float z00 = z[0], z01 = m01 ? z[1] : 0.0f, z10 = m10 ? z[B.zw[0]] : 0.0f,
+                  z11 = m01 && m10 ? z[B.zw[0] + 1] : 0.0f, d = B.dd[k];
+      const float wt = (f & UF_Y ? 0.5f : 1.0f) * (f & UF_X ? 0.5f : 1.0f);
+      const float pz = __fmul_rn(wt, __fadd_rn(__fadd_rn(__fadd_rn(z00, z01), z10), z11));
+      m = d > 0.0f ? fmaf(d, __fadd_rn(B.rp[k], B.sp[k]), pz) : 0.0f;
+    }
+    B.mt[k] = m;
+  }
+  __syncthreads();
+  for (int k = tid; k < B.np; k += PT) {
+    float z = 0.0f;
+    if (B.uf[k] & UF_RING) {
+      const float* const m = B.mt + k;
+      const float d = B.dd[k];
+      const float acc = __fadd_rn(B.rp[k], __fadd_rn(__fadd_rn(m[-1], m[1]), __fadd_rn(m[-W], m[W])));
+      z = d > 0.0f ? fmaf(d, acc, __fmul_rn(W_KEEP, m[0])) : 0.0f;
+    }
+    B.m2[k] = z;
+  }
+  __syncthreads();
+  for (int k = tid; k < B.np; k += PT) {
+    const int j = B.dj[k];
+    if (j < DJ_OWN) continue;
+    const float* const m = B.m2 + k;
+    const float d = B.dd[k];
+    const float sm = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(0.0f, m[-1]), m[1]), m[-W]), m[W]);
+    __stcg(a.z32 + (j - DJ_OWN), d > 0.0f ? fmaf(W_KEEP, m[0], __fmul_rn(d, __fadd_rn(B.rp[k], sm))) : 0.0f);
   }
 }
 
@@ -1239,7 +1345,7 @@ __device__ __forceinline__ void coarse_rows(const PoissonArgs& a, const FusedBlo
       }
       for (; j < nc; j += 32) s0 = fmaf(row[j], rcs[j], s0);
     };
-    if (t < a.crows) dot(B.crow + (size_t)t * nc);
+    if (t < B.crows) dot(B.crow + (size_t)t * nc);
     else dot(a.cinv + (size_t)k * nc);
     float s = (s0 + s1) + (s2 + s3);
 #pragma unroll
@@ -1273,7 +1379,9 @@ __device__ __forceinline__ double picard_update(const PoissonArgs& a, int i) {
   return V;
 }
 
+template <bool RUNS>
 __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
+  constexpr int NVB = RUNS ? FUSED_NVB_RUNS : FUSED_NVB_MAX, PATCH = RUNS ? FUSED_PATCH : FUSED_PATCH + 1;
   extern __shared__ float4 dyn_smem[];
   float* rcs = reinterpret_cast<float*>(dyn_smem);
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1292,7 +1400,7 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
 
   __shared__ FusedLevel lv[MG_MAX_LEVELS];
   FusedBlock B;
-  fused_tables(a, c0, c1, B, lv);
+  fused_tables<RUNS>(a, c0, c1, B, lv);
   __syncthreads();
   const int nc = __ldg(a.nc_dev);
   int ci[2], zi = -1;
@@ -1340,6 +1448,7 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
     const double inner_at_pic = n_inner, outer_at_pic = n_outer;
     // the Picard update of the solve before, the right-hand side, the residual.  The update
     // writes x off the free nodes only, which no residual reads.
+    float rv[2] = {0.0f, 0.0f};  // this thread's residuals
     if (act) {
       double ff = 0.0, rr = 0.0;
 #pragma unroll 1
@@ -1355,6 +1464,7 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
         __stcg(a.f + i, fi);
         ff = fma(fi, fi, ff);
         const double res = DSUB(fi, apply_d(o, i));
+        (o ? rv[1] : rv[0]) = (float)res;
         __stcg(a.r32 + i, (float)res);
         rr = fma(res, res, rr);
       }
@@ -1363,7 +1473,7 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
     }
     grid_barrier(a);
     double norm2[2];
-    VwTotal<2>(a, slot++).sums(a, norm2);
+    VwTotal<2, NVB>(a, slot++).sums(a, norm2);
     const double fnorm2 = norm2[0];
     double rnorm2 = norm2[1];
     tmark(a, 17);
@@ -1377,7 +1487,7 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
         const int j = B.dj[k];
         B.rp[k] = j >= 0 ? *(a.r32 + (j & ~DJ_OWN)) : 0.0f;
       }
-      down_tile(a, B);
+      down_tile<RUNS>(a, B);
       grid_barrier(a);
       tmark(a, 0);
       for (int k = 0; k < a.max_inner; ++k) {
@@ -1397,7 +1507,7 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
         coarse_rows(a, B, rcs, nc, ci, zi);
         grid_barrier(a);
         tmark(a, 7);
-        for (int l = last - 1; l >= (a.join1 ? 2 : 1); --l) {
+        for (int l = last - 1; l >= 2; --l) {
           const MgLevel &F = lv[l].L, &C = lv[l + 1].L;
           const int* const yx = lv[l].yx;
           for (int q = tid; q < lv[l].share; q += PT)
@@ -1408,32 +1518,43 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
           grid_barrier(a);
           tmark(a, 8 + (l < 7 ? l : 6));
         }
-        float zo[2], rv[2];
-        up_runs(a, B, lv, in, 32 * warp + lane, zo, rv);
+        float zo[2], zn[2][4];
+        auto neighbours = [&]() {
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            const float* const z = a.z32 + 32 * c + lane + o * nv;
+            const int f = code[o];
+            zn[o][0] = f & 1 ? *(z - 1) : 0.0f;
+            zn[o][1] = f & 2 ? *(z + 1) : 0.0f;
+            zn[o][2] = f & 4 ? *(z - nx) : 0.0f;
+            zn[o][3] = f & 8 ? *(z + nx) : 0.0f;
+          }
+        };
+        if (RUNS) {
+          up_runs(a, B, lv, in, 32 * warp + lane, zo);
+#pragma unroll
+          for (int o = 0; o < 2; ++o)
+            if (in[o]) __stcg(a.z32 + 32 * c + lane + o * nv, zo[o]);
+        } else {
+          up_tile(a, B);
+          grid_barrier(a);
+          tmark(a, 9);
+#pragma unroll
+          for (int o = 0; o < 2; ++o) zo[o] = in[o] ? *(a.z32 + 32 * c + lane + o * nv) : 0.0f;
+          neighbours();
+        }
         if (act) {
           double rz_p = 0.0;
 #pragma unroll
-          for (int o = 0; o < 2; ++o) {
-            if (!in[o]) continue;
-            __stcg(a.z32 + 32 * c + lane + o * nv, zo[o]);
-            rz_p += (double)rv[o] * (double)zo[o];
-          }
+          for (int o = 0; o < 2; ++o)
+            if (in[o]) rz_p += (double)rv[o] * (double)zo[o];
           vw_put(a, slot, 0, part, rz_p);
         }
         grid_barrier(a);
         tmark(a, 8);
         // p = z + beta p, q = A p
-        VwTotal<1> tz(a, slot++);
-        float zn[2][4];
-#pragma unroll
-        for (int o = 0; o < 2; ++o) {
-          const float* const z = a.z32 + 32 * c + lane + o * nv;
-          const int f = code[o];
-          zn[o][0] = f & 1 ? *(z - 1) : 0.0f;
-          zn[o][1] = f & 2 ? *(z + 1) : 0.0f;
-          zn[o][2] = f & 4 ? *(z - nx) : 0.0f;
-          zn[o][3] = f & 8 ? *(z + nx) : 0.0f;
-        }
+        VwTotal<1, NVB> tz(a, slot++);
+        if (RUNS) neighbours();
         const double rz = tz.sum(a);
         const float beta = (float)(k == 0 ? 0.0 : rz / rz_old);
         if (act) {
@@ -1454,34 +1575,36 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
         tmark(a, 14);
         // e += alpha p, r -= alpha q (on the nodes and on the tile's patch), then the next
         // V-cycle's restrictions
-        VwTotal<1> tq(a, slot++);
-        float qp[FUSED_PATCH];
+        VwTotal<1, NVB> tq(a, slot++);
+        float qp[PATCH];
 #pragma unroll
-        for (int e = 0; e < FUSED_PATCH; ++e) {
+        for (int e = 0; e < PATCH; ++e) {
           const int t = tid + e * PT, j = t < B.np ? B.dj[t] : -1;
           qp[e] = j >= 0 ? *(a.q32 + (j & ~DJ_OWN)) : 0.0f;
         }
         const double pq = tq.sum(a);
         const float al = (float)(pq != 0.0 ? rz / pq : 0.0);
 #pragma unroll
-        for (int e = 0; e < FUSED_PATCH; ++e) {
+        for (int e = 0; e < PATCH; ++e) {
           const int t = tid + e * PT;
           if (t < B.np) B.rp[t] = fmaf(-al, qp[e], B.rp[t]);
         }
+        for (int t = tid + PATCH * PT; t < B.np; t += PT)
+          if (B.dj[t] >= 0) B.rp[t] = fmaf(-al, *(a.q32 + (B.dj[t] & ~DJ_OWN)), B.rp[t]);
         if (act) {
           double rr_p = 0.0;
 #pragma unroll
           for (int o = 0; o < 2; ++o) {
             rv[o] = fmaf(-al, qv[o], rv[o]);
             ev[o] = fmaf(al, pv[o], ev[o]);
-            if (in[o]) __stcg(a.r32 + 32 * c + lane + o * nv, rv[o]);
+            if (RUNS && in[o]) __stcg(a.r32 + 32 * c + lane + o * nv, rv[o]);
             rr_p += (double)rv[o] * (double)rv[o];
           }
           vw_put(a, slot, 0, part, rr_p);
         }
-        down_tile(a, B);
+        down_tile<RUNS>(a, B);
         grid_barrier(a);
-        const double rrk = VwTotal<1>(a, slot++).sum(a);
+        const double rrk = VwTotal<1, NVB>(a, slot++).sum(a);
         tmark(a, 15);
         rz_old = rz;
         if (rrk <= a.tol_inner * a.tol_inner * rr0 || rrk <= target2) break;  // as in poisson_body
@@ -1500,13 +1623,14 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
           const int i = 32 * c + lane + o * nv;
           if (!(code[o] & 128)) continue;
           const double res = DSUB((*(a.f + i)), apply_d(o, i));
-          __stcg(a.r32 + i, (float)res);
+          rv[o] = (float)res;
+          __stcg(a.r32 + i, rv[o]);
           rr = fma(res, res, rr);
         }
         vw_put(a, slot, 0, part, rr);
       }
       grid_barrier(a);
-      rnorm2 = VwTotal<1>(a, slot++).sum(a);
+      rnorm2 = VwTotal<1, NVB>(a, slot++).sum(a);
       tmark(a, 16);
     }
     if (!(rnorm2 <= target2) && fnorm2 > 0.0 && gbid(a) == 0 && tid == 0) atomicOr(a.errflags, PB_EF_POISSON_NOCONV);
@@ -1525,8 +1649,11 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
 }
 
 __global__ void __launch_bounds__(PT, 1) k_poisson(const __grid_constant__ PoissonArgs a) { poisson_body(a); }
-__global__ void __launch_bounds__(PT, 1) k_poisson_fused(const __grid_constant__ PoissonArgs a) {
-  poisson_body_fused(a);
+__global__ void __launch_bounds__(PT, 1) k_poisson_runs(const __grid_constant__ PoissonArgs a) {
+  poisson_body_fused<true>(a);
+}
+__global__ void __launch_bounds__(PT, 1) k_poisson_tiles(const __grid_constant__ PoissonArgs a) {
+  poisson_body_fused<false>(a);
 }
 
 __global__ void __launch_bounds__(PT, 1) k_poisson_batch(const PoissonArgs* __restrict__ args,

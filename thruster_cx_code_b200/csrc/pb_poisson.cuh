@@ -66,8 +66,7 @@ struct PoissonArgs {
   double* partials;       // 4 slots x 2 values x nvb doubles
   int fused;              // joined phases (fused_plan)
   int dt_y, dt_x;         // tiles of level 2 of the joined restriction, one per block
-  int join1;              // level 1's up leg is computed with the fine one's
-  int crows;              // rows of the coarse inverse that a block keeps in shared memory
+  int croom;              // room (floats) for rows of the coarse inverse in shared memory
   double* wpart;          // 4 slots x 2 values x 32 nvb doubles: warp sums of the virtual blocks
   unsigned int* bar;      // barrier word, zero at launch (its low bits must start at zero)
   uint32_t* errflags;
@@ -184,23 +183,22 @@ inline void fine_up_tiles(int ny, int nx, int nblk, int* ty_out, int* tx_out) {
   *tx_out = btx;
 }
 
-// Joined phases (k_poisson_fused).  fused_plan lays out the restriction's tiles of level 2, one
-// per block (the smallest patch of level 0), and the shared memory behind the coarse
+// Joined phases (k_poisson_runs, k_poisson_tiles).  fused_plan lays out the restriction's tiles of
+// level 2, one per block (the smallest patch of level 0), and the shared memory behind the coarse
 // right-hand side: the tables and patches of FusedBlock, then as many of the block's rows of
 // the coarse inverse as fit.  smem is 0 where the solve takes the general kernel: periodic grids
-// (a level's wrap is not the finer level's), fewer than three levels, more than two passes of
-// the virtual blocks or fewer blocks than virtual blocks (a warp keeps one virtual warp's
-// nodes in registers), and grids too large for the shared memory: above about 100,000 nodes,
-// where a phase is no longer all latency.
-constexpr int FUSED_HALO = 11;      // patch of level 0 under h rows of level 2: 4 h + 11
-constexpr int FUSED_PATCH = 3;      // patch nodes per thread
-constexpr int FUSED_JOIN = 1200;    // level-1 nodes under a block's runs (join1)
-constexpr int FUSED_NVB_MAX = 74;
-constexpr size_t FUSED_SMEM_MAX = 200 * 1024;
+// (a level's wrap is not the finer level's), fewer than three levels, more than two nodes a
+// thread of the virtual blocks or fewer blocks than virtual blocks (a warp keeps one virtual
+// warp's nodes in registers), patches too large for the shared memory.
+constexpr int FUSED_HALO = 11, FUSED_HALO_TILE = 15;  // patch of level 0 under h rows of level 2: 4 h + this
+constexpr int FUSED_PATCH = 3;      // patch nodes per thread whose update is loaded ahead
+constexpr int FUSED_RUN = 128;      // longest run that the up leg takes by runs
+constexpr int FUSED_NVB_RUNS = 32, FUSED_NVB_MAX = 148;
+constexpr size_t FUSED_SMEM_MAX = 206 * 1024;
 
 struct FusedPlan {
   size_t smem = 0;
-  int ty = 1, tx = 1, join1 = 0, crows = 0;
+  int runs = 0, ty = 1, tx = 1, croom = 0;
 };
 
 inline FusedPlan fused_plan(const MgLevel* lev, int nlevels, bool periodic, int nu0, int max_inner, int nvb, int nblk,
@@ -209,29 +207,35 @@ inline FusedPlan fused_plan(const MgLevel* lev, int nlevels, bool periodic, int 
   if (periodic || nu0 != 2 || nlevels < 3 || max_inner < 1 || nvb > FUSED_NVB_MAX || nblk < nvb) return p;
   const int ny = lev[0].ny, nx = lev[0].nx, ny2 = lev[2].ny, nx2 = lev[2].nx;
   if ((long)ny * nx > 2048L * nvb || 4L * ny2 < ny || 4L * nx2 < nx || ny > 32767 || nx > 32767) return p;
-  long best = -1, floats = 0;
-  for (int ty = 1; ty <= ny2 && ty <= nblk; ++ty) {
-    const int tx = std::min(nx2, nblk / ty);
-    const long h = (ny2 + ty - 1) / ty, w = (nx2 + tx - 1) / tx, patch = (4 * h + FUSED_HALO) * (4 * w + FUSED_HALO);
-    if (best >= 0 && patch >= best) continue;
-    best = patch;
-    floats = 4 * patch + 3 * (2 * h + 3) * (2 * w + 3) + 27 * h * w;
-    p.ty = ty;
-    p.tx = tx;
-  }
-  if (best > 1024L * FUSED_PATCH) return p;
-  const long run = 32L * ((32L * nvb + nblk - 1) / nblk);
-  if (run > nx) return p;
-  // a run's rows of level 1: at most four of (run + 6) / 2 + 2 nodes for each of two segments
-  const long nz = 2 * 4 * ((run + 13) / 2 + 6);
-  p.join1 = nz <= FUSED_JOIN;
-  floats += 6 * 10 * (run + 4) + (p.join1 ? 20 : 2) * nz;
+  long levels = 0;
   for (int l = 1; l < nlevels; ++l)
-    floats += 32 * ((((long)lev[l].ny * lev[l].nx + 31) / 32 + nblk - 1) / nblk);
-  const long room = (long)FUSED_SMEM_MAX / 4 - floats;
-  if (room < 0) return p;
-  p.crows = (int)std::min<long>((ncap + nblk - 1) / nblk, room / std::max(ncap, 1));
-  p.smem = 4 * (size_t)(floats + (long)p.crows * ncap);
+    levels += 32 * ((((long)lev[l].ny * lev[l].nx + 31) / 32 + nblk - 1) / nblk);
+  const long rows = (long)ncap * ((ncap + nblk - 1) / nblk), max_floats = (long)FUSED_SMEM_MAX / 4;
+  for (int runs = 1; runs >= 0; --runs) {
+    const long halo = runs ? FUSED_HALO : FUSED_HALO_TILE, halo1 = runs ? 3 : 5;
+    long best = -1, floats = 0;
+    for (int ty = 1; ty <= ny2 && ty <= nblk; ++ty) {
+      const int tx = std::min(nx2, nblk / ty);
+      const long h = (ny2 + ty - 1) / ty, w = (nx2 + tx - 1) / tx, patch = (4 * h + halo) * (4 * w + halo);
+      if (best >= 0 && patch >= best) continue;
+      best = patch;
+      floats = (runs ? 4 : 6) * patch + 3 * (2 * h + halo1) * (2 * w + halo1) + 27 * h * w;
+      if (!runs) floats += 20 * (2 * h + 3) * (2 * w + 3) + 2 * (h + 4) * (w + 4);
+      p.ty = ty;
+      p.tx = tx;
+    }
+    floats += levels;
+    if (runs) {
+      const long run = 32L * ((32L * nvb + nblk - 1) / nblk), nz = 2 * 4 * ((run + 13) / 2 + 6);
+      if (nvb > FUSED_NVB_RUNS || run > FUSED_RUN || run > nx || best > 1024L * FUSED_PATCH) continue;
+      floats += 6 * 10 * (run + 4) + 20 * nz;
+    }
+    if (floats > max_floats) continue;
+    p.runs = runs;
+    p.croom = (int)std::min(rows, max_floats - floats);
+    p.smem = 4 * (size_t)(floats + p.croom);
+    break;
+  }
   return p;
 }
 
@@ -241,7 +245,9 @@ inline FusedPlan fused_plan(const MgLevel* lev, int nlevels, bool periodic, int 
 // tolerance, not bit for bit, unlike the particle arithmetic.
 // One instance on every block of the launch.
 __global__ void k_poisson(const __grid_constant__ PoissonArgs a);
-__global__ void k_poisson_fused(const __grid_constant__ PoissonArgs a);
+// One instance with joined phases (fused_plan).
+__global__ void k_poisson_runs(const __grid_constant__ PoissonArgs a);
+__global__ void k_poisson_tiles(const __grid_constant__ PoissonArgs a);
 // Several instances in one launch: block b runs the instances listed at blk_map[blk_map[b]]
 // (a count, then indices into args) one after another, each together with the other blocks of
 // its contiguous range (args[i].blk0, args[i].nblk): an instance with blocks of its own, or

@@ -586,8 +586,7 @@ static void set_up_tiles(Sim* s, PoissonArgs* a) {
   a->fused = s->fu.smem > 0;
   a->dt_y = s->fu.ty;
   a->dt_x = s->fu.tx;
-  a->join1 = s->fu.join1;
-  a->crows = s->fu.crows;
+  a->croom = s->fu.croom;
 }
 
 static PoissonArgs poisson_args(Sim* s, int iterations, const pb_step_params* p) {
@@ -674,7 +673,8 @@ static int32_t launch_poisson(Sim* s, int iterations, const pb_step_params* p) {
   }
   PoissonArgs a = poisson_args(s, iterations, p);
   void* args[] = {&a};
-  if (a.fused) return coop_field_launch(s, (const void*)k_poisson_fused, args, 16 * (size_t)a.vb_off + s->fu.smem);
+  if (a.fused)
+    return coop_field_launch(s, s->fu.runs ? (const void*)k_poisson_runs : (const void*)k_poisson_tiles, args, 16 * (size_t)a.vb_off + s->fu.smem);
   return coop_field_launch(s, (const void*)k_poisson, args, mg_solve_smem_bytes(s->ncap, a.nvb, a.nblk));
 }
 
@@ -1218,7 +1218,7 @@ static uint64_t state_signature(const pb_sim* h) {
   k = fnv(k, ptrs, sizeof(ptrs));
   for (const DevLevel& L : s->lev) k = fnv_v(k, L);
   const long long vals[] = {s->ny, s->nx, s->periodic, s->ngrids, s->nc, s->trace_on, s->pgrid, s->ut[0], s->ut[1],
-                            s->fu.ty, s->fu.tx, s->fu.join1, s->fu.crows, (long long)s->fu.smem,
+                            s->fu.ty, s->fu.tx, s->fu.runs, s->fu.croom, (long long)s->fu.smem,
                             s->pbps, s->ppb, (long long)s->kopts, (long long)s->psmem, (long long)s->tile_cap, s->see_cap,
                             s->angle_cap, (long long)s->sort_cap, (long long)s->hist_cap, s->counts_valid ? 1 : 0,
                             s->max_outer, s->max_inner, s->nu, h->cx.nt, h->see.nt, s->profiling, s->ncap,
@@ -1363,8 +1363,9 @@ int32_t pb_sim_create(pb_sim** out, int32_t device) {
                           (int)mg_solve_smem_bytes(MG_MAX_COARSE, s->num_sms, 1)));
   CK(cudaFuncSetAttribute((const void*)k_poisson, cudaFuncAttributePreferredSharedMemoryCarveout,
                           (int)cudaSharedmemCarveoutMaxL1));
-  CK(cudaFuncSetAttribute((const void*)k_poisson_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)(16 * (size_t)mg_vb_offset(MG_MAX_COARSE) + FUSED_SMEM_MAX)));
+  for (const void* k : {(const void*)k_poisson_runs, (const void*)k_poisson_tiles})
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)(16 * (size_t)mg_vb_offset(MG_MAX_COARSE) + FUSED_SMEM_MAX)));
   s->pgrid = s->num_sms;
   CK(dalloc(&s->partials, 4 * 2 * (size_t)s->num_sms));
   CK(dalloc(&s->wpart, 4 * 2 * 32 * (size_t)FUSED_NVB_MAX));
