@@ -671,6 +671,7 @@ int32_t pb_batch_run(pb_batch* b, pb_sim* const* sims, int32_t n, const pb_step_
     for (int k = 0; k < K; ++k)
       if ((rc = check_step_params(&sims[i]->s, &params[(size_t)i * K + k]))) return rc;
   bool use_graphs = b->graphs_on != 0;
+  for (int i = 0; i < n; ++i) sims[i]->s.breaks_none = false;
   for (int i = 0; i < n; ++i)
     if (sims[i]->s.profiling || sims[i]->s.trace_on) use_graphs = false;
   if (use_graphs) {

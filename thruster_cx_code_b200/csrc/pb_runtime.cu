@@ -200,6 +200,9 @@ struct Sim {
   int* mg_dirty = nullptr;
   uint32_t* mg_status = nullptr;
   bool erosion_seen = false;     // a step with sputter breaks was enqueued: field solves rebuild first
+  bool breaks_none = false;      // no cell broke since the hierarchy was last rebuilt (reports read say so)
+  bool rebuild_enqueued = false; // k_mg_rebuild was enqueued since pb_sim_step cleared this
+  bool bar_zeroed = false;       // this step's reset zeroed the barrier word
   long long mg_host_rebuilds = 0;
   double *partials = nullptr, *wpart = nullptr;
   unsigned int* bar = nullptr;
@@ -245,6 +248,8 @@ struct Sim {
   // report
   pb_step_report* rep_dev = nullptr;
   pb_step_report* rep_host = nullptr;
+  bool report_direct = false;  // k_step_end writes the report to rep_host (pb_sim_step)
+  unsigned int* end_ticket = nullptr;
   pb_step_report* rep_run = nullptr;  // pinned per-step reports of pb_sim_run
   int rep_run_cap = 0;
   // settings
@@ -541,6 +546,7 @@ static int32_t build_operator(Sim* s, const uint8_t* isBound_host) {
   CK(cudaMemcpy(s->nc_dev, &s->nc, sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemset(s->mg_dirty, 0, sizeof(int)));
   CK(cudaMemset(s->mg_status, 0, sizeof(uint32_t)));
+  s->breaks_none = true;
   return PB_OK;
 }
 
@@ -648,7 +654,9 @@ static int32_t coop_launch(int device, cudaStream_t st, Launch launch) {
 // simulator's own stream (a graph runs its simulator alone, so no other cooperative launch
 // is chained against it), otherwise through the device's chain.
 static int32_t coop_field_launch(Sim* s, const void* kernel, void** args, size_t smem) {
-  CK(cudaMemsetAsync(s->bar, 0, 2 * sizeof(unsigned int), s->stream));
+  // a step's reset has zeroed the barrier word, and whole barriers leave its low bits at zero (a
+  // memset between two kernels is 4 us of the step)
+  if (!s->bar_zeroed) CK(cudaMemsetAsync(s->bar, 0, 2 * sizeof(unsigned int), s->stream));
   if (s->capturing) {
     CK(cudaLaunchCooperativeKernel(kernel, dim3(s->pgrid), dim3(PT), args, smem, s->stream));
   } else {
@@ -664,9 +672,12 @@ static int32_t coop_field_launch(Sim* s, const void* kernel, void** args, size_t
 static int32_t launch_poisson(Sim* s, int iterations, const pb_step_params* p) {
   if (iterations <= 0) return PB_OK;
   int32_t rc;
-  if (s->erosion_seen) {
+  if (s->erosion_seen && !s->breaks_none) {
     // cells may have broken since the last solve: the hierarchy follows the node classes
-    // first (k_mg_rebuild returns at once unless a break set mg_dirty)
+    // first (k_mg_rebuild returns at once unless a break set mg_dirty; its launch alone is
+    // 6 us of a step, left out when every report since the last rebuild has been read and
+    // names no broken cell)
+    s->rebuild_enqueued = true;
     MgRebuildArgs m = mg_rebuild_args(s);
     void* margs[] = {&m};
     if ((rc = coop_field_launch(s, (const void*)k_mg_rebuild, margs, 0))) return rc;
@@ -690,6 +701,7 @@ struct StepResetArgs {
   unsigned long long* tile_status;
   long long ntile;
   int *angle_count, *see_count, *see_spawned, *tile_counter, *ni_dst, *ne_dst, *inj;
+  unsigned int* bar;
   unsigned long long* ds_bits;
 };
 
@@ -707,6 +719,7 @@ __global__ void __launch_bounds__(256) k_step_reset(const __grid_constant__ Step
       a.ds_bits[0] = 0ull; a.ds_bits[1] = 0ull; a.ds_bits[2] = 0ull;
       a.tile_counter[0] = 0; a.tile_counter[1] = 0;
       *a.ni_dst = 0; *a.ne_dst = 0;
+      a.bar[0] = a.bar[1] = 0u;
     }
     __syncthreads();  // the counts' error flags are words of the report
     if (threadIdx.x < 32) inject_counts(inject);
@@ -739,6 +752,10 @@ struct StepEndArgs {
   int n_saddle;
   SaddleIdx sidx;
   const uint32_t* mg_status;
+  // the report's copy in pinned host memory, written by the block that ends last (a copy
+  // operation behind the kernel is 10 us of the step), or null
+  uint32_t* host;
+  unsigned int* ticket;
   float* angles;
   const int* angle_count;
   int angle_cap;
@@ -753,11 +770,28 @@ struct StepEndArgs {
   double* accum;
 };
 
+__device__ __forceinline__ void step_report_out(const StepEndArgs& a) {
+  if (!a.host) return;
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1;  // back to zero after the last
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  constexpr int nw = (int)(sizeof(pb_step_report) / 4) + 1;  // the rebuild's status past it
+  const uint32_t* const r = reinterpret_cast<const uint32_t*>(a.r);
+  for (int i = threadIdx.x; i < nw; i += blockDim.x) a.host[i] = __ldcg(r + i);
+}
+
 __global__ void __launch_bounds__(STEP_END_NT) k_step_end(const __grid_constant__ StepEndArgs a) {
   pdl_enter();
   if (blockIdx.x > 0) {
     node_stats(a.T, a.Tnext, a.isBound, a.gridmask, a.ngrids, a.r->grid_sums, a.ppc, a.accum,
                (unsigned long long*)&a.r->ppc_active, a.N, (int)blockIdx.x - 1, (int)gridDim.x - 1);
+    step_report_out(a);
     return;
   }
   pb_step_report* const r = a.r;
@@ -789,6 +823,7 @@ __global__ void __launch_bounds__(STEP_END_NT) k_step_end(const __grid_constant_
     default: break;
   }
   theta95(a.angles, a.angle_count, a.angle_cap, a.angle_scratch, &r->theta95);
+  step_report_out(a);
 }
 
 }  // namespace pb
@@ -971,8 +1006,10 @@ static int32_t enqueue_step_pre(pb_sim* h, const pb_step_params* p) {
     r.tile_status = s->tile_status; r.ntile = 2 * (long long)s->tile_cap;
     r.angle_count = s->angle_count; r.see_count = s->see_count; r.see_spawned = s->see_spawned;
     r.ds_bits = s->ds_bits; r.tile_counter = s->tile_counter; r.ni_dst = ni_dst; r.ne_dst = ne_dst; r.inj = s->inj;
+    r.bar = s->bar;
     CK(launch_pdl(k_step_reset, 1 + grid_for(s, std::max<long>(N, 2 * (long)s->tile_cap), 256), 256, 0, st, r, ia));
     ++s->launches;
+    s->bar_zeroed = true;
   }
 
   // RF co-extraction: V_fixed on one grid, then recalc_poisson(2) (:984-991)
@@ -1147,6 +1184,8 @@ static int32_t enqueue_step_post(pb_sim* h, const pb_step_params* p) {
   ea.ci = I.cur; ea.ce = E.cur; ea.ds_bits = s->ds_bits; ea.V = s->V; ea.pstats = s->pstats;
   ea.n_saddle = std::max(0, std::min(p->n_saddle, 8));
   for (int k = 0; k < 8; ++k) ea.sidx.v[k] = p->saddle_idx[k];
+  ea.host = s->report_direct ? reinterpret_cast<uint32_t*>(s->rep_host) : nullptr;
+  ea.ticket = s->end_ticket;
   ea.mg_status = s->mg_status; ea.angles = s->angles; ea.angle_count = s->angle_count; ea.angle_cap = s->angle_cap;
   ea.angle_scratch = s->angle_scratch;
   ea.N = N; ea.ngrids = std::min(s->ngrids, 16); ea.T = s->Tmap; ea.Tnext = p->thermal_on ? s->Tnext : nullptr;
@@ -1162,6 +1201,7 @@ static int32_t enqueue_step_post(pb_sim* h, const pb_step_params* p) {
     if ((rc = sort_species(s, 0, bits))) return rc;
     if ((rc = sort_species(s, 1, bits))) return rc;
   }
+  s->bar_zeroed = false;  // a solve outside a step zeroes the word itself
   mark(s);
   CK(cudaGetLastError());
   return PB_OK;
@@ -1222,7 +1262,7 @@ static uint64_t state_signature(const pb_sim* h) {
                             s->pbps, s->ppb, (long long)s->kopts, (long long)s->psmem, (long long)s->tile_cap, s->see_cap,
                             s->angle_cap, (long long)s->sort_cap, (long long)s->hist_cap, s->counts_valid ? 1 : 0,
                             s->max_outer, s->max_inner, s->nu, h->cx.nt, h->see.nt, s->profiling, s->ncap,
-                            s->max_coarse, s->erosion_seen ? 1 : 0};
+                            s->max_coarse, s->erosion_seen ? 1 : 0, s->breaks_none ? 1 : 0, s->report_direct ? 1 : 0};
   k = fnv(k, vals, sizeof(vals));
   const double dv[] = {s->tol, s->tol_inner, h->cx.lo, h->cx.hi, h->cx.cmax, h->see.lo, h->see.hi};
   k = fnv(k, dv, sizeof(dv));
@@ -1333,8 +1373,6 @@ static int32_t run_one_step(pb_sim* h, const pb_step_params* p) {
 
 // the report and, past it, the rebuild's status (k_step_end)
 static int32_t finish_report(Sim* s, pb_step_report* out, uint32_t* mg_status) {
-  CK(cudaMemcpyAsync(s->rep_host, s->rep_dev, sizeof(pb_step_report) + sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                     s->stream));
   CK(cudaStreamSynchronize(s->stream));
   *out = *s->rep_host;
   std::memcpy(mg_status, s->rep_host + 1, sizeof(uint32_t));
@@ -1393,6 +1431,8 @@ int32_t pb_sim_create(pb_sim** out, int32_t device) {
   CK(dalloc(&s->see_xy, 2 * (size_t)s->see_cap));
   CK(dalloc(&s->angles, (size_t)s->angle_cap));
   CK(dalloc(&s->angle_scratch, 2 * (size_t)s->angle_cap));
+  CK(dalloc(&s->end_ticket, 1));
+  CK(cudaMemset(s->end_ticket, 0, sizeof(unsigned int)));
   CK(dalloc(&s->rep_dev, 2));  // the report and the words past it (k_step_end)
   CK(cudaMemset(s->rep_dev, 0, 2 * sizeof(pb_step_report)));
   CK(dalloc(&s->step_dev, 1));
@@ -1427,7 +1467,7 @@ int32_t pb_sim_destroy(pb_sim* h) {
                s->tile_status, s->tile_counter, s->see_key, s->see_count, s->angle_scratch, s->angle_count,
                s->ds_bits, s->n_sub, s->inj, s->see_spawned, s->skey[0], s->skey[1], s->sval[0], s->sval[1],
                s->shist, s->sblk, s->rep_dev, h->cx.t, h->cx.c, h->see.t, h->see.c, s->solve_ns, s->nc_dev,
-               s->mg_counts, s->mg_dirty, s->mg_status, s->ptrace};
+               s->mg_counts, s->mg_dirty, s->mg_status, s->ptrace, s->end_ticket};
   for (void* q : v) if (q) cudaFree(q);
   for (int k = 0; k < 2; ++k)
     for (int b = 0; b < 2; ++b) {
@@ -1917,7 +1957,13 @@ int32_t pb_sim_step(pb_sim* h, const pb_step_params* p, pb_step_report* report) 
   s->mark_used = 0;
   s->launches = 0;
   CK(cudaEventRecord(s->ev0, s->stream));
-  if ((rc = run_one_step(h, p))) return rc;
+  const bool none = s->breaks_none || !s->erosion_seen;
+  s->rebuild_enqueued = false;
+  s->report_direct = report != nullptr;
+  rc = run_one_step(h, p);
+  s->report_direct = false;
+  s->breaks_none = false;
+  if (rc) return rc;
   CK(cudaEventRecord(s->ev1, s->stream));
   if (report) {
     uint32_t status = 0;
@@ -1925,6 +1971,7 @@ int32_t pb_sim_step(pb_sim* h, const pb_step_params* p, pb_step_report* report) 
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
     s->last_ms = ms;
+    s->breaks_none = (none || s->rebuild_enqueued) && report->broken == 0;
     if ((rc = settle_mg(s, &status))) return rc;
   }
   return PB_OK;
@@ -1950,7 +1997,9 @@ int32_t pb_sim_run(pb_sim* h, const pb_step_params* params, int32_t nsteps, pb_s
   s->launches = 0;
   CK(cudaEventRecord(s->ev0, s->stream));
   for (int k = 0; k < nsteps; ++k) {
-    if ((rc = run_one_step(h, &params[k]))) return rc;
+    rc = run_one_step(h, &params[k]);
+    s->breaks_none = false;
+    if (rc) return rc;
     if (reports) {
       CK(cudaMemcpyAsync(&s->rep_run[k], s->rep_dev, sizeof(pb_step_report), cudaMemcpyDeviceToHost, s->stream));
     }
