@@ -546,8 +546,10 @@ __global__ void __launch_bounds__(256) k_thermal_taichi(const float* __restrict_
 
 // ------------------------------------------------------------------ cell-key radix sort
 // Stable LSD radix sort of (key, index) pairs, RADIX_BITS per pass; identical permutation
-// to np.argsort(key, kind="stable").  Three kernels per pass: tile digit histograms,
-// a digit-major exclusive scan, and a stable scatter (warp-ordered ranks).
+// to np.argsort(key, kind="stable").  Per pass: tile digit histograms, a digit-major exclusive
+// scan, and a stable scatter.  A thread's elements of a tile are loaded at once and ranked by
+// its warp alone (one block barrier instead of three for every 256 elements, and one exposed
+// load instead of eight): a pass of 80k particles 44 -> 22 us, of 6M 95 -> 62, of 48M 820 -> 700.
 __global__ void k_sort_keys(const float* x, const float* y, const int* n_dev, int nx, int ny, float dxf, float dyf,
                             uint32_t* key, uint32_t* val) {
   pdl_enter();
@@ -558,60 +560,38 @@ __global__ void k_sort_keys(const float* x, const float* y, const int* n_dev, in
   }
 }
 
+constexpr int SORT_PER = SORT_TILE / SORT_NT;  // elements per thread: warp w takes SORT_PER chunks of 32 in a row
+
 __global__ void __launch_bounds__(SORT_NT) k_sort_hist(const uint32_t* key, const int* n_dev, int shift,
                                                        uint32_t* hist, int ntiles) {
   pdl_enter();
   __shared__ uint32_t h[RADIX];
-  int n = *n_dev;
+  const int n = *n_dev, tile = blockIdx.x, lane = threadIdx.x & 31;
+  const int i0 = tile * SORT_TILE + (int)(threadIdx.x >> 5) * (32 * SORT_PER) + lane;
+  uint32_t k[SORT_PER];
+#pragma unroll
+  for (int e = 0; e < SORT_PER; ++e) k[e] = i0 + 32 * e < n ? (key[i0 + 32 * e] >> shift) & (RADIX - 1) : RADIX;
   for (int d = threadIdx.x; d < RADIX; d += blockDim.x) h[d] = 0;
   __syncthreads();
-  int tile = blockIdx.x;
-  int t0 = tile * SORT_TILE;
-  for (int k = threadIdx.x; k < SORT_TILE; k += blockDim.x) {
-    int i = t0 + k;
-    if (i < n) atomicAdd(&h[(key[i] >> shift) & (RADIX - 1)], 1u);
+  // where neighbours agree (sorted keys, their high digits) the lanes of one digit add once:
+  // 32 adds to one word take turns; scattered digits add one by one, which a match would slow
+  // (143 us against 83 on 48M keys in upload order)
+#pragma unroll
+  for (int e = 0; e < SORT_PER; ++e) {
+    const uint32_t left = __shfl_up_sync(0xFFFFFFFFu, k[e], 1);
+    if (__popc(__ballot_sync(0xFFFFFFFFu, left == k[e])) >= 8) {
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, k[e]);
+      if (k[e] < RADIX && (peers & ((1u << lane) - 1)) == 0) atomicAdd(&h[k[e]], (uint32_t)__popc(peers));
+    } else if (k[e] < RADIX) {
+      atomicAdd(&h[k[e]], 1u);
+    }
   }
   __syncthreads();
   for (int d = threadIdx.x; d < RADIX; d += blockDim.x) hist[(size_t)d * ntiles + tile] = h[d];
 }
 
-// exclusive scan of hist (RADIX * ntiles, digit-major) in one block
-__global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* hist, int total) {
-  pdl_enter();
-  __shared__ uint32_t carry;
-  __shared__ uint32_t sm[32];
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < total; c0 += blockDim.x) {
-    int i = c0 + threadIdx.x;
-    uint32_t v = i < total ? hist[i] : 0u;
-    uint32_t inc = v;
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-      if (lane >= o) inc += t;
-    }
-    if (lane == 31) sm[w] = inc;
-    __syncthreads();
-    if (w == 0) {
-      uint32_t s = lane < (int)(blockDim.x >> 5) ? sm[lane] : 0u;
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xFFFFFFFFu, s, o);
-        if (lane >= o) s += t;
-      }
-      sm[lane] = s;
-    }
-    __syncthreads();
-    uint32_t ex = carry + (w ? sm[w - 1] : 0u) + inc - v;
-    if (i < total) hist[i] = ex;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += sm[(blockDim.x >> 5) - 1];
-    __syncthreads();
-  }
-}
-
-// Multi-block exclusive scan of a long uint32 array: per-chunk sums, a one-block scan of
-// the sums (k_sort_scan), then each chunk scanned from its base.
+// Multi-block exclusive scan of a long uint32 array: per-chunk sums (only when there are several
+// chunks), then each chunk scanned from the sum of those before it, which its block adds.
 constexpr int SCAN_NT = 1024, SCAN_PER = 8, SCAN_CHUNK = SCAN_NT * SCAN_PER;
 
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total) {
@@ -639,14 +619,26 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
   return ex;
 }
 
+// this thread's SCAN_PER values of a chunk, zero past the end
+__device__ __forceinline__ void scan_load(const uint32_t* a, int total, int base, uint32_t (&v)[SCAN_PER]) {
+  if (base + SCAN_PER <= total) {
+#pragma unroll
+    for (int k = 0; k < SCAN_PER; k += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(a + base + k);  // a from cudaMalloc, base a multiple of 8
+      v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < SCAN_PER; ++k) v[k] = base + k < total ? a[base + k] : 0u;
+  }
+}
+
 __global__ void __launch_bounds__(SCAN_NT) k_scan_partials(const uint32_t* a, int total, uint32_t* bsum) {
   pdl_enter();
-  const int base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_PER;
-  uint32_t s = 0u;
+  uint32_t v[SCAN_PER], s = 0u, t;
+  scan_load(a, total, blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_PER, v);
 #pragma unroll
-  for (int k = 0; k < SCAN_PER; ++k)
-    if (base + k < total) s += a[base + k];
-  uint32_t t;
+  for (int k = 0; k < SCAN_PER; ++k) s += v[k];
   block_excl_scan(s, &t);
   if (threadIdx.x == 0) bsum[blockIdx.x] = t;
 }
@@ -654,14 +646,15 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_partials(const uint32_t* a, in
 __global__ void __launch_bounds__(SCAN_NT) k_scan_apply(uint32_t* a, int total, const uint32_t* bsum) {
   pdl_enter();
   const int base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_PER;
-  uint32_t v[SCAN_PER];
-  uint32_t s = 0u;
-#pragma unroll
-  for (int k = 0; k < SCAN_PER; ++k) {
-    v[k] = base + k < total ? a[base + k] : 0u;
-    s += v[k];
+  uint32_t v[SCAN_PER], s = 0u, before = 0u, first = 0u;
+  scan_load(a, total, base, v);
+  if (blockIdx.x > 0) {
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += SCAN_NT) before += bsum[b];
+    block_excl_scan(before, &first);
   }
-  uint32_t ex = block_excl_scan(s, nullptr) + bsum[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < SCAN_PER; ++k) s += v[k];
+  uint32_t ex = block_excl_scan(s, nullptr) + first;
 #pragma unroll
   for (int k = 0; k < SCAN_PER; ++k) {
     if (base + k < total) a[base + k] = ex;
@@ -669,46 +662,54 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_apply(uint32_t* a, int total, 
   }
 }
 
-// stable scatter: within a tile, elements are ranked per digit in index order
+// stable scatter: each warp ranks its elements per digit in index order, then the digits'
+// counts are summed over the warps before it
 __global__ void __launch_bounds__(SORT_NT) k_sort_scatter(const uint32_t* key, const uint32_t* val, const int* n_dev,
                                                           int shift, const uint32_t* offs, int ntiles,
                                                           uint32_t* key_out, uint32_t* val_out) {
   pdl_enter();
-  __shared__ uint32_t base[RADIX];
-  __shared__ uint32_t wcount[SORT_NT / 32][RADIX];
-  int n = *n_dev;
-  int tile = blockIdx.x;
-  int t0 = tile * SORT_TILE;
-  for (int d = threadIdx.x; d < RADIX; d += blockDim.x) base[d] = offs[(size_t)d * ntiles + tile];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int NW = SORT_NT / 32;
-  // process the tile in rounds of SORT_NT consecutive elements (index order)
-  for (int r0 = 0; r0 < SORT_TILE; r0 += SORT_NT) {
-    for (int d = lane; d < RADIX; d += 32) wcount[w][d] = 0;
-    __syncthreads();
-    int i = t0 + r0 + threadIdx.x;
-    bool v = i < n;
-    uint32_t k = v ? key[i] : 0u;
-    uint32_t d = (k >> shift) & (RADIX - 1);
-    unsigned peers = __match_any_sync(0xFFFFFFFFu, v ? d : 0xFFFFFFFFu);
-    int rank_in_warp = __popc(peers & ((1u << lane) - 1));
-    if (v && rank_in_warp == 0) wcount[w][d] = __popc(peers);
-    __syncthreads();
-    if (v) {
-      uint32_t before = 0;
-      for (int q = 0; q < w; ++q) before += wcount[q][d];
-      uint32_t pos = base[d] + before + rank_in_warp;
-      key_out[pos] = k;
-      val_out[pos] = val[i];
+  constexpr int NW = SORT_NT / 32;
+  __shared__ uint32_t count[NW][RADIX];
+  const int n = *n_dev, tile = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i0 = tile * SORT_TILE + w * (32 * SORT_PER) + lane;
+  uint32_t k[SORT_PER], v[SORT_PER], r[SORT_PER];
+#pragma unroll
+  for (int e = 0; e < SORT_PER; ++e) {
+    const bool in = i0 + 32 * e < n;
+    k[e] = in ? key[i0 + 32 * e] : 0u;
+    v[e] = in ? val[i0 + 32 * e] : 0u;
+  }
+  static_assert(RADIX <= SORT_NT, "one thread per digit");
+  const uint32_t off = threadIdx.x < RADIX ? offs[(size_t)threadIdx.x * ntiles + tile] : 0u;
+  for (int d = lane; d < RADIX; d += 32) count[w][d] = 0u;
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < SORT_PER; ++e) {
+    const bool in = i0 + 32 * e < n;
+    const uint32_t d = (k[e] >> shift) & (RADIX - 1);
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, in ? d : RADIX), before = peers & ((1u << lane) - 1);
+    r[e] = in ? count[w][d] + __popc(before) : 0u;
+    __syncwarp();
+    if (in && before == 0) count[w][d] += __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  if (threadIdx.x < RADIX) {
+    uint32_t at = off;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) {
+      const uint32_t c = count[q][threadIdx.x];
+      count[q][threadIdx.x] = at;
+      at += c;
     }
-    __syncthreads();
-    // advance digit bases by this round's counts
-    for (int dd = threadIdx.x; dd < RADIX; dd += blockDim.x) {
-      uint32_t s = 0;
-      for (int q = 0; q < NW; ++q) s += wcount[q][dd];
-      base[dd] += s;
-    }
-    __syncthreads();
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < SORT_PER; ++e) {
+    if (i0 + 32 * e >= n) continue;
+    const uint32_t pos = count[w][(k[e] >> shift) & (RADIX - 1)] + r[e];
+    key_out[pos] = k[e];
+    val_out[pos] = v[e];
   }
 }
 

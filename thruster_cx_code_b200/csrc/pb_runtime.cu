@@ -866,10 +866,12 @@ static int32_t sort_perm(Sim* s, int k, int ncell_bits, const uint32_t** perm) {
     ++s->launches;
     {
       const int total = RADIX * ntiles, nb = (total + SCAN_CHUNK - 1) / SCAN_CHUNK;
-      CK(launch_pdl(k_scan_partials, nb, SCAN_NT, 0, st, s->shist, total, s->sblk));
-      CK(launch_pdl(k_sort_scan, 1, 1024, 0, st, s->sblk, nb));
+      if (nb > 1) {
+        CK(launch_pdl(k_scan_partials, nb, SCAN_NT, 0, st, s->shist, total, s->sblk));
+        ++s->launches;
+      }
       CK(launch_pdl(k_scan_apply, nb, SCAN_NT, 0, st, s->shist, total, s->sblk));
-      s->launches += 3;
+      ++s->launches;
     }
     CK(launch_pdl(k_sort_scatter, ntiles, SORT_NT, 0, st, s->skey[a], s->sval[a], n_src, shift, s->shist, ntiles,
                                                 s->skey[1 - a], s->sval[1 - a]));
