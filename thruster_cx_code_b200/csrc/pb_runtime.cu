@@ -1942,6 +1942,7 @@ int32_t pb_sim_poisson(pb_sim* h, int32_t iterations, const pb_step_params* p, d
   Sim* s = &h->s;
   if (!s->domain_set) return fail(PB_ERR_STATE, "pb_sim_poisson: no domain");
   CK(cudaMemsetAsync(&s->rep_dev->errflags, 0, sizeof(uint32_t), s->stream));
+  s->bar_zeroed = false;  // also after a step that failed half enqueued
   int32_t rc = launch_poisson(s, iterations, p);
   if (rc) return rc;
   uint32_t f = 0;
