@@ -1,4 +1,4 @@
-"""set_particles below and above the size from which its parts run as a pipeline: particles,
+"""set_particles, whose parts run as a pipeline: particles,
 order, flags and next id against a stable argsort of the same cell keys, from pageable and
 pinned arrays."""
 import numpy as np

@@ -273,7 +273,7 @@ struct Sim {
   float *pw_vals = nullptr, *pw_out = nullptr;
   size_t pw_cap_leaves = 0, pw_cap_nodes = 0, pw_cap_h = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  // large uploads (pb_sim_upload_particles): their copies' stream, made at the first one
+  // uploads (pb_sim_upload_particles): their copies' stream, made at the first one
   cudaStream_t up = nullptr;
   cudaEvent_t ev_up = nullptr;
   uint32_t* up_max = nullptr;
@@ -1700,12 +1700,13 @@ int32_t pb_sim_set_particles(pb_sim* h, int32_t species, int32_t n, const float*
   return PB_OK;
 }
 
-// From this many particles an upload runs as a pipeline: its copies on a stream of their own, the
-// cell keys sorted while the other arrays are on their way, each array re-ordered behind its own
-// copy (a gather by itself keeps more of its source in L2 than one of all arrays), the largest id
-// found on the device.  UPLOAD_FIGURES
-constexpr int UPLOAD_PIPE_MIN = 1 << 20;
-
+// An upload runs as a pipeline: its copies on a stream of their own, the cell keys sorted while the
+// other arrays are on their way, each array re-ordered behind its own copy (a gather by itself
+// keeps more of its source in L2 than one of all arrays), the largest id found on the device.
+// Pinned arrays of n ions on 129 x 568 nodes, queued on one stream / so (single runs, 10% apart):
+// 100k 248 / 173 us, 250k 417 / 464, 500k 795 / 724, 1M 1143 / 892, 2M 1303 / 1362, 4M 2459 / 2043,
+// 16M 9908 / 7375; 48M ions and 16M electrons 59 ms as
+// copies, largest id on the host and sort one after another, 33 ms so (the copies alone 28.6).
 static int32_t upload_piped(Sim* s, int k, int n, const float* const* f, const uint8_t* cex, const uint32_t* id,
                             int bits, uint32_t* top) {
   if (!s->up) CK(cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking));
@@ -1761,26 +1762,6 @@ static int32_t upload_piped(Sim* s, int k, int n, const float* const* f, const u
   return PB_OK;
 }
 
-static int32_t upload_plain(Sim* s, int k, int n, const float* const* f, const uint8_t* cex, const uint32_t* id,
-                            int bits, uint32_t* top) {
-  Species& S = s->sp[k];
-  const Soa& b = S.buf[S.cur];
-  const size_t n4 = (size_t)n * 4;
-  float* const dst[5] = {b.x, b.y, b.vx, b.vy, b.vz};
-  for (int a = 0; a < 5; ++a) CK(cudaMemcpyAsync(dst[a], f[a], n4, cudaMemcpyHostToDevice, s->stream));
-  CK(cudaMemcpyAsync(b.id, id, n4, cudaMemcpyHostToDevice, s->stream));
-  if (S.ion) {
-    if (cex) CK(cudaMemcpyAsync(b.cex, cex, n, cudaMemcpyHostToDevice, s->stream));
-    else CK(cudaMemsetAsync(b.cex, 0, n, s->stream));
-  }
-  int32_t rc;
-  if (bits && (rc = sort_species(s, k, bits))) return rc;
-  uint32_t m = 0;
-  for (int i = 0; i < n; ++i) m = std::max(m, id[i]);
-  *top = m;
-  return PB_OK;
-}
-
 int32_t pb_sim_upload_particles(pb_sim* h, int32_t species, int32_t n, const float* x, const float* y, const float* vx,
                                 const float* vy, const float* vz, const uint8_t* cex, const uint32_t* id,
                                 int64_t min_next_id, int32_t sort, double dx, double dy, int64_t* next_id) {
@@ -1806,7 +1787,7 @@ int32_t pb_sim_upload_particles(pb_sim* h, int32_t species, int32_t n, const flo
   CK(cudaMemcpyAsync(s->counts + 2 * species + S.cur, &n, sizeof(int), cudaMemcpyHostToDevice, s->stream));
   if (n > 0) {
     const float* const f[5] = {x, y, vx, vy, vz};
-    rc = (n >= UPLOAD_PIPE_MIN ? upload_piped : upload_plain)(s, species, n, f, cex, id, bits, &top);
+    rc = upload_piped(s, species, n, f, cex, id, bits, &top);
     // the caller's arrays are read and the particles in place when this returns, and nothing
     // reads the arrays any more if it failed
     const cudaError_t e = s->up ? cudaStreamSynchronize(s->up) : cudaSuccess;
