@@ -350,7 +350,8 @@ __global__ void __launch_bounds__(THERMAL_NT) k_thermal(const float* T, float* T
   __shared__ uint8_t M[TW * TW];
   const int gx0 = blockIdx.x * TT - HALO, gy0 = blockIdx.y * TT - HALO;
   float c[PER];
-  unsigned flags[PER];  // bits 0-3: the neighbour left, right, down, up is bound; 4: swept; 5: bound; 6: output
+  // bits 0-3: the neighbour left, right, down, up is bound; 4: swept; 5: a mask cell; 6: output; 7: bound
+  unsigned flags[PER];
   int found = 0;
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
@@ -373,7 +374,8 @@ __global__ void __launch_bounds__(THERMAL_NT) k_thermal(const float* T, float* T
         found = 1;
       }
       c[j] = t;
-      if (m & 1) flags[j] |= 32u;
+      // a mask cell of an even value is cooled only; node_stats moves it as every mask cell
+      flags[j] = (m ? 32u : 0u) | (m & 1) << 7;
       if ((m & 1) && gy >= 1 && gy <= ny - 2 && gx >= 1 && gx <= nx - 2 && ly >= 1 && ly <= TW - 2 && lx >= 1 &&
           lx <= TW - 2)
         flags[j] |= 16u;
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(THERMAL_NT) k_thermal(const float* T, float* T
     const int k = threadIdx.x + j * THERMAL_NT;
     const int ly = k / TW, lx = k - ly * TW;
     const float v = c[j];
-    Tnext[(size_t)(gy0 + ly) * nx + gx0 + lx] = (v != v) ? v : (v > 300.0f ? v : 300.0f);
+    Tnext[(size_t)(gy0 + ly) * nx + gx0 + lx] = (v != v || !(flags[j] & 128u)) ? v : (v > 300.0f ? v : 300.0f);
   }
 }
 
