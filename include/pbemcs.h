@@ -67,7 +67,7 @@ int32_t pb_accumulate_rho_noalloc(const float* x, const float* y, float* rho, in
 
 /* pb_push_particles_boris (large calls), pb_accumulate_rho and pb_compute_particle_substeps
  * take their scratch from a stream-ordered memory pool of the library's own, which keeps up to
- * 256 MB per context between calls.  This gives what is not in use back to the device. */
+ * 352 MB per context between calls.  This gives what is not in use back to the device. */
 int32_t pb_release_scratch(void);
 
 /* Exhaustive check of the division the step kernels use for x / dx and y / dy (no

@@ -47,7 +47,11 @@ static int32_t fail(int32_t code, const std::string& msg) {
 // threads never share memory that is in use.  A capturing stream, and anything unexpected,
 // takes the default pool as before.  pb_release_scratch gives unused memory back, and so does
 // an allocation of the simulator's own that finds the device full.
-constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
+// What is kept covers the largest scratch of one call, the packed push's corners (80 bytes a
+// cell), with room for a count map beside it: with 256 MB kept, a packed push on 4.2M cells that
+// is waited for took 1002 us (8M particles; 224 us back to back, 488 us unpacked), now 217 us.
+constexpr long long PUSH_PACK_CELLS = 4ll << 20;  // cells of the largest grid that the push packs
+constexpr uint64_t SCRATCH_KEEP = (uint64_t)PUSH_PACK_CELLS * 80 + (32ull << 20);  // 352 MB
 struct ScratchPool {
   unsigned long long ctx = 0;
   cudaMemPool_t pool = nullptr;
@@ -2258,7 +2262,6 @@ int32_t pb_release_scratch(void) {
 
 // Where pb_push_particles_boris packs the corners first
 constexpr int PUSH_PACK_MIN = 600000;
-constexpr long long PUSH_PACK_CELLS = 4ll << 20;  // at most 320 MB of corners
 
 int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float* vz, const float* Ex, const float* Ey,
                                 const float* Bx, const float* By, const float* Bz, int32_t num_p, double dx, double dy,
