@@ -205,7 +205,7 @@ struct Sim {
   uint32_t* mg_status = nullptr;
   bool erosion_seen = false;     // a step with sputter breaks was enqueued: field solves rebuild first
   bool breaks_none = false;      // no cell broke since the hierarchy was last rebuilt (reports read say so)
-  bool rebuild_enqueued = false; // k_mg_rebuild was enqueued since pb_sim_step cleared this
+  bool rebuild_enqueued = false; // k_mg_rebuild was enqueued, or replayed, since pb_sim_step cleared this
   bool bar_zeroed = false;       // this step's reset zeroed the barrier word
   long long mg_host_rebuilds = 0;
   double *partials = nullptr, *wpart = nullptr;
@@ -298,6 +298,7 @@ struct Sim {
     uint64_t pkey = 0, skey = 0;   // parameter digest, state signature before the step
     cudaGraphExec_t exec = nullptr;
     long long launches = 0;
+    bool rebuilds = false;         // holds a launch of k_mg_rebuild
   };
   std::vector<StepGraph> graphs;
   long long graph_captures = 0, graph_replays = 0, graph_plain_steps = 0;
@@ -1309,6 +1310,7 @@ static int32_t graph_step(pb_sim* h, const pb_step_params* p, bool* done) {
     s->sp_dx = p->dx;
     s->sp_dy = p->dy;
     if (p->erosion_on) s->erosion_seen = true;
+    if (g.rebuilds) s->rebuild_enqueued = true;
     s->launches += g.launches;
     s->step_dev_val = (long long)(uint32_t)p->iteration + 1;
     ++s->graph_replays;
@@ -1320,7 +1322,7 @@ static int32_t graph_step(pb_sim* h, const pb_step_params* p, bool* done) {
   const int cur0 = s->sp[0].cur, cur1 = s->sp[1].cur;
   const bool cv0 = s->counts_valid;
   const double dx0 = s->sp_dx, dy0 = s->sp_dy;
-  const bool es0 = s->erosion_seen;
+  const bool es0 = s->erosion_seen, re0 = s->rebuild_enqueued;
   const long long l0 = s->launches;
   if (s->graphs.size() >= 8) free_graphs(s);
   cudaError_t ce = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
@@ -1331,6 +1333,7 @@ static int32_t graph_step(pb_sim* h, const pb_step_params* p, bool* done) {
     return PB_OK;
   }
   s->capturing = 1;
+  s->rebuild_enqueued = false;
   int32_t rc = enqueue_step(h, p);
   if (rc == PB_OK) {
     k_step_advance<<<1, 1, 0, s->stream>>>(s->step_dev);
@@ -1349,6 +1352,7 @@ static int32_t graph_step(pb_sim* h, const pb_step_params* p, bool* done) {
     cudaGetLastError();
     s->sp[0].cur = cur0; s->sp[1].cur = cur1;
     s->counts_valid = cv0; s->sp_dx = dx0; s->sp_dy = dy0; s->erosion_seen = es0; s->launches = l0;
+    s->rebuild_enqueued = re0;
     return PB_OK;
   }
   Sim::StepGraph g;
@@ -1356,6 +1360,8 @@ static int32_t graph_step(pb_sim* h, const pb_step_params* p, bool* done) {
   g.skey = skey;
   g.exec = exec;
   g.launches = s->launches - l0 + 1;
+  g.rebuilds = s->rebuild_enqueued;
+  s->rebuild_enqueued = re0 || g.rebuilds;
   s->launches = l0 + g.launches;
   s->graphs.push_back(g);
   CK(cudaGraphLaunch(exec, s->stream));
