@@ -539,7 +539,8 @@ __global__ void __launch_bounds__(256) k_thermal_taichi(const float* __restrict_
       reinterpret_cast<float4*>(Tn)[q] = v;
     }
   }
-  for (int i = done + t0; i < N; i += stride) {
+  for (unsigned e = (unsigned)done + t0; e < (unsigned)N; e += stride) {  // may end above 2^31
+    const int i = (int)e;
     const float c = T[i];
     const int iy = i / nx, ix = i - iy * nx;
     Tn[i] = __ldg(mask + i) == 1 ? taichi_cell(T, mask, i, iy, ix, nx, ny, c, Fo_x, Fo_y) : c;

@@ -395,11 +395,13 @@ __device__ __forceinline__ int substep_count(double ds_max, double ds_lim, uint3
 }
 
 // ------------------------------------------------------------------ standalone push
+// The module kernels' indexes past the last whole vector are unsigned: a count may be close to
+// 2^31, and the index that ends a loop is up to a grid's threads above it.
 __global__ void k_push_boris(float* x, float* y, float* vx, float* vy, float* vz, const float* Ex,
                              const float* Ey, const float* Bx, const float* By, const float* Bz, int n,
                              int nx, int ny, float dxf, float dyf, double h, float dtf) {
   pdl_enter();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)n; i += gridDim.x * blockDim.x) {
     float a = x[i], b = y[i], c = vx[i], d = vy[i], e = vz[i];
     boris_push_one<true>(a, b, c, d, e, Ex, Ey, Bx, By, Bz, nx, ny, dxf, dyf, h, dtf);
     x[i] = a; y[i] = b; vx[i] = c; vy[i] = d; vz[i] = e;
@@ -519,7 +521,7 @@ __global__ void __launch_bounds__(256, 4) k_push_corner(float* __restrict__ x, f
       reinterpret_cast<float4*>(vz)[q] = W;
     }
   }
-  for (int i = done + t0; i < n; i += stride) {
+  for (unsigned i = (unsigned)done + t0; i < (unsigned)n; i += stride) {
     float a = x[i], b = y[i], c = vx[i], d = vy[i], e = vz[i];
     push_corner_one<HAS_B>(a, b, c, d, e, Ec, Bc, nx, ny, dxf, dyf, h, dtf, rc);
     x[i] = a; y[i] = b; vx[i] = c; vy[i] = d; vz[i] = e;
@@ -633,9 +635,9 @@ __global__ void __launch_bounds__(256) k_count_cells(const float* __restrict__ x
       count_add(cnt, c3, v);
     }
   }
-  for (int i0 = done + t0 - (threadIdx.x & 31); i0 < n; i0 += stride) {
-    const int i = i0 + (threadIdx.x & 31);
-    const bool v = i < n;
+  for (unsigned i0 = (unsigned)done + t0 - (threadIdx.x & 31); i0 < (unsigned)n; i0 += stride) {
+    const unsigned i = i0 + (threadIdx.x & 31);
+    const bool v = i < (unsigned)n;
     count_add(cnt, v ? deposit_cell(x[i], y[i], dxf, dyf, nx, ny) : 0, v);
   }
 }
@@ -693,7 +695,7 @@ __global__ void __cluster_dims__(DEP_C, 1, 1) __launch_bounds__(1024)
       if (r < n4) { add(Z.x, W.x); add(Z.y, W.y); add(Z.z, W.z); add(Z.w, W.w); }
     }
   }
-  for (int i = done + t0; i < n; i += stride) add(x[i], y[i]);
+  for (unsigned i = (unsigned)done + t0; i < (unsigned)n; i += stride) add(x[i], y[i]);
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   const uint32_t base = smem_addr(hist);
   uint32_t at[DEP_C];
@@ -867,7 +869,7 @@ __device__ __forceinline__ void substep_block(const float* __restrict__ x, const
       m = b > m ? b : m;
     }
   }
-  for (int i = 4 * n4 + t0; i < n; i += stride) {
+  for (unsigned i = 4u * n4 + t0; i < (unsigned)n; i += stride) {
     double ds = predicted_ds(x[i], y[i], vx[i], vy[i], vz[i], Ex, Ey, Ec, nx, ny, dxf, dyf, qm, dtf, dt2, inv_dx, inv_dy);
     unsigned long long b = (unsigned long long)__double_as_longlong(ds);
     m = b > m ? b : m;
@@ -955,7 +957,7 @@ __global__ void k_segment_hits(const uint8_t* isBound, int nx, int ny, float dxf
                                const float* y0, const float* x1, const float* y1, int n, uint8_t* hit,
                                int64_t* hix, int64_t* hiy) {
   pdl_enter();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)n; i += gridDim.x * blockDim.x) {
     SegHit s = segment_hit(isBound, nx, ny, dxf, dyf, x0[i], y0[i], x1[i], y1[i]);
     hit[i] = s.hit;
     hix[i] = s.ix;

@@ -2315,7 +2315,7 @@ int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float*
     }
     cudaGetLastError();  // no memory for the corners: the push without them
   }
-  int g = (int)std::min<long>((num_p + bs - 1) / bs, 148L * 16);
+  int g = (int)std::min<long>((num_p + (long)bs - 1) / bs, 148L * 16);
   k_push_boris<<<g, bs, 0, st>>>(x, y, vx, vy, vz, Ex, Ey, Bx, By, Bz, num_p, nx, ny, (float)dx, (float)dy, h, (float)dt);
   CK(cudaGetLastError());
   return PB_OK;
@@ -2451,7 +2451,7 @@ int32_t pb_thermal_conduction(const float* T, float* T_new, const int32_t* mask,
   const bool vec = (((uintptr_t)T | (uintptr_t)T_new | (uintptr_t)mask) & 15u) == 0;
   const int per = vec ? 4 : 1;
   CK(launch_pdl(vec ? k_thermal_taichi<true> : k_thermal_taichi<false>,
-                (int)std::min<long>((G / per + 256) / 256, 148L * 16), 256, 0, (cudaStream_t)stream, T, T_new, mask, nx, ny,
+                (int)std::min<long>((G / per + 256L) / 256, 148L * 16), 256, 0, (cudaStream_t)stream, T, T_new, mask, nx, ny,
                 (float)Fo_x, (float)Fo_y));
   return PB_OK;
 }
@@ -2474,7 +2474,7 @@ int32_t pb_compute_particle_substeps(const float* x, const float* y, const float
   unsigned* ebound = reinterpret_cast<unsigned*>(bits + 1);
   const int gc = (int)std::min<long long>((G + 255) / 256, 148LL * 8);
   k_e_corners<<<gc, 256, 0, st>>>(Ex, Ey, ec, ny, nx, ebound);
-  int g = (int)std::min<long>((n + 255) / 256, 148L * 16);
+  int g = (int)std::min<long>((n + 255L) / 256, 148L * 16);
   k_substep_reduce<<<g, 256, 0, st>>>(x, y, vx, vy, vz, n, Ex, Ey, ec, nx, ny, (float)dx, (float)dy, qm,
                                       (float)dt, dt * dt, bits, ebound);
   unsigned long long hb = 0;
@@ -2495,7 +2495,7 @@ int32_t pb_segment_hits_grid(const uint8_t* isBound, int32_t nx, int32_t ny, dou
                              const float* y0, const float* x1, const float* y1, int32_t n, uint8_t* hit,
                              int64_t* hit_ix, int64_t* hit_iy, void* stream) {
   if (n <= 0) return PB_OK;
-  int g = (int)std::min<long>((n + 255) / 256, 148L * 16);
+  int g = (int)std::min<long>((n + 255L) / 256, 148L * 16);
   k_segment_hits<<<g, 256, 0, (cudaStream_t)stream>>>(isBound, nx, ny, (float)dx, (float)dy, x0, y0, x1, y1, n, hit,
                                                        hit_ix, hit_iy);
   CK(cudaGetLastError());
