@@ -1684,13 +1684,20 @@ int32_t pb_sim_reserve(pb_sim* h, int32_t species, int32_t capacity) {
   return alloc_species(s, species, capacity, s->host_num[species]);
 }
 
+// storage for n particles and a quarter more
+static int32_t room_for(Sim* s, int k, int n) {
+  const long long cap = (long long)n + n / 4 + 4096;
+  if (cap > INT32_MAX - 1023) return fail(PB_ERR_CAPACITY, "more particles than a species can hold");  // whole 1024s
+  return alloc_species(s, k, (int)cap, 0);
+}
+
 int32_t pb_sim_set_particles(pb_sim* h, int32_t species, int32_t n, const float* x, const float* y, const float* vx,
                              const float* vy, const float* vz, const uint8_t* cex, const uint32_t* id,
                              uint32_t next_id) {
   Sim* s = &h->s;
   if (species < 0 || species > 1 || n < 0) return fail(PB_ERR_ARG, "pb_sim_set_particles");
   int32_t rc;
-  if ((rc = alloc_species(s, species, std::max(n + n / 4 + 4096, 4096), 0))) return rc;
+  if ((rc = room_for(s, species, n))) return rc;
   Species& S = s->sp[species];
   Soa& b = S.buf[S.cur];
   size_t n4 = (size_t)n * 4;
@@ -1779,7 +1786,7 @@ int32_t pb_sim_upload_particles(pb_sim* h, int32_t species, int32_t n, const flo
   if (species < 0 || species > 1 || n < 0 || !next_id || (n > 0 && (!x || !y || !vx || !vy || !vz || !id)))
     return fail(PB_ERR_ARG, "pb_sim_upload_particles");
   int32_t rc;
-  if ((rc = alloc_species(s, species, std::max(n + n / 4 + 4096, 4096), 0))) return rc;
+  if ((rc = room_for(s, species, n))) return rc;
   Species& S = s->sp[species];
   const bool sorted = sort && n > 0;
   const int32_t order = !sorted ? PB_OK
