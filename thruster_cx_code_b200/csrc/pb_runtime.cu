@@ -1717,6 +1717,19 @@ int32_t pb_sim_set_particles(pb_sim* h, int32_t species, int32_t n, const float*
   return PB_OK;
 }
 
+// The device `d` for a scope, the caller's own after it.
+struct DeviceScope {
+  int was = -1, d;
+  cudaError_t err;
+  explicit DeviceScope(int dev) : d(dev) {
+    err = cudaGetDevice(&was);
+    if (err == cudaSuccess && was != d) err = cudaSetDevice(d);
+  }
+  ~DeviceScope() {
+    if (was >= 0 && was != d) cudaSetDevice(was);
+  }
+};
+
 // An upload runs as a pipeline: its copies on a stream of their own, the cell keys sorted while the
 // other arrays are on their way, each array re-ordered behind its own copy (a gather by itself
 // keeps more of its source in L2 than one of all arrays), the largest id found on the device.
@@ -1785,6 +1798,10 @@ int32_t pb_sim_upload_particles(pb_sim* h, int32_t species, int32_t n, const flo
   Sim* s = &h->s;
   if (species < 0 || species > 1 || n < 0 || !next_id || (n > 0 && (!x || !y || !vx || !vy || !vz || !id)))
     return fail(PB_ERR_ARG, "pb_sim_upload_particles");
+  // the copies' stream and event and the launches belong to the simulator's device, whichever
+  // the calling thread has selected
+  const DeviceScope dev(s->device);
+  CK(dev.err);
   int32_t rc;
   if ((rc = room_for(s, species, n))) return rc;
   Species& S = s->sp[species];
