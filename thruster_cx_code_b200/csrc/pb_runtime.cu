@@ -705,7 +705,7 @@ struct StepResetArgs {
   int N;
   unsigned long long* tile_status;
   long long ntile;
-  int *angle_count, *see_count, *see_spawned, *tile_counter, *ni_dst, *ne_dst, *inj;
+  int *angle_count, *see_count, *see_spawned, *tile_counter, *ni_dst, *ne_dst;
   unsigned int* bar;
   unsigned long long* ds_bits;
 };
@@ -713,7 +713,6 @@ struct StepResetArgs {
 __global__ void __launch_bounds__(256) k_step_reset(const __grid_constant__ StepResetArgs a,
                                                     const __grid_constant__ InjectArgs inject) {
   pdl_enter();
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long long)gridDim.x * blockDim.x;
   static_assert(sizeof(pb_step_report) % 4 == 0 && offsetof(pb_step_report, ppc_min) % 4 == 0, "report words");
   constexpr int nw = (int)(sizeof(pb_step_report) / 4), w0 = (int)(offsetof(pb_step_report, ppc_min) / 4);
   if (blockIdx.x == 0) {
@@ -728,9 +727,11 @@ __global__ void __launch_bounds__(256) k_step_reset(const __grid_constant__ Step
     }
     __syncthreads();  // the counts' error flags are words of the report
     if (threadIdx.x < 32) inject_counts(inject);
-    if (gridDim.x > 1) return;
+    return;
   }
-  const long long first = gridDim.x > 1 ? tid - blockDim.x : tid, step = gridDim.x > 1 ? nth - blockDim.x : nth;
+  // the other blocks (the launch has two or more)
+  const long long first = (long long)(blockIdx.x - 1) * blockDim.x + threadIdx.x;
+  const long long step = (long long)(gridDim.x - 1) * blockDim.x;
   for (long long i = first; i < a.N; i += step) a.ppc[i] = 0;
   for (long long i = first; i < a.ntile; i += step) a.tile_status[i] = 0ull;
 }
@@ -1012,7 +1013,7 @@ static int32_t enqueue_step_pre(pb_sim* h, const pb_step_params* p) {
     r.rep = rep; r.ppc = s->ppc; r.N = N;
     r.tile_status = s->tile_status; r.ntile = 2 * (long long)s->tile_cap;
     r.angle_count = s->angle_count; r.see_count = s->see_count; r.see_spawned = s->see_spawned;
-    r.ds_bits = s->ds_bits; r.tile_counter = s->tile_counter; r.ni_dst = ni_dst; r.ne_dst = ne_dst; r.inj = s->inj;
+    r.ds_bits = s->ds_bits; r.tile_counter = s->tile_counter; r.ni_dst = ni_dst; r.ne_dst = ne_dst;
     r.bar = s->bar;
     CK(launch_pdl(k_step_reset, 1 + grid_for(s, std::max<long>(N, 2 * (long)s->tile_cap), 256), 256, 0, st, r, ia));
     ++s->launches;
