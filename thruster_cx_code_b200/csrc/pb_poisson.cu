@@ -636,6 +636,31 @@ __device__ __forceinline__ void solve_end(const PoissonArgs& a, int tid, int nth
   }
 }
 
+// V_new of node i from the solution, then the damped Picard update
+__device__ __forceinline__ double picard_update(const PoissonArgs& a, int i) {
+  const uint8_t c = __ldg(a.cls + i);
+  double vn;
+  if (c == NC_FREE) vn = (*(a.x + i));
+  else if (c == NC_DIR) vn = __ldg(a.Vfixed + i);
+  else {
+    int y = i / a.nx, x = i - y * a.nx;
+    int sy = y, sx = x;
+    if (x == a.nx - 1) {
+      sx = x - 1;  // right: copy (y, nx-2), which may itself be a top/bottom copy
+      uint8_t cs = __ldg(a.cls + sy * a.nx + sx);
+      if (cs == NC_NEU && !a.periodic) sy = (sy == 0) ? 1 : (sy == a.ny - 1 ? a.ny - 2 : sy);
+    } else if (y == 0) sy = 1;
+    else sy = a.ny - 2;
+    int j = sy * a.nx + sx;
+    uint8_t cj = __ldg(a.cls + j);
+    vn = (cj == NC_DIR) ? __ldg(a.Vfixed + j) : (*(a.x + j));
+  }
+  if (c != NC_FREE) __stcg(a.x + i, vn);
+  const double V = DADD(DMUL(a.omega_keep, (*(a.V + i))), DMUL(a.omega_new, vn));
+  __stcg(a.V + i, V);
+  return V;
+}
+
 // ----------------------------------------------------------------- the persistent kernel
 __device__ __forceinline__ void poisson_body(const PoissonArgs& a) {
   extern __shared__ float4 dyn_smem[];
@@ -812,28 +837,7 @@ __device__ __forceinline__ void poisson_body(const PoissonArgs& a) {
     last_rel = fnorm2 > 0.0 ? sqrt(rnorm2 / fnorm2) : 0.0;
 
     // ---- V_new on every node, then the damped Picard update
-    for (int i = tid; i < N; i += nth) {
-      uint8_t c = __ldg(a.cls + i);
-      double vn;
-      if (c == NC_FREE) vn = (*(a.x + i));
-      else if (c == NC_DIR) vn = __ldg(a.Vfixed + i);
-      else {
-        int y = i / a.nx, x = i - y * a.nx;
-        int sy = y, sx = x;
-        if (x == a.nx - 1) {
-          sx = x - 1;  // right: copy (y, nx-2), which may itself be a top/bottom copy
-          uint8_t cs = __ldg(a.cls + sy * a.nx + sx);
-          if (cs == NC_NEU && !a.periodic) sy = (sy == 0) ? 1 : (sy == a.ny - 1 ? a.ny - 2 : sy);
-        } else if (y == 0) sy = 1;
-        else sy = a.ny - 2;
-        int j = sy * a.nx + sx;
-        uint8_t cj = __ldg(a.cls + j);
-        vn = (cj == NC_DIR) ? __ldg(a.Vfixed + j) : (*(a.x + j));
-      }
-      if (c != NC_FREE) __stcg(a.x + i, vn);
-      double Vi = (*(a.V + i));
-      __stcg(a.V + i, DADD(DMUL(a.omega_keep, Vi), DMUL(a.omega_new, vn)));
-    }
+    for (int i = tid; i < N; i += nth) picard_update(a, i);
     grid_barrier(a);
     tmark(a, 18);
   }
@@ -1352,31 +1356,6 @@ __device__ __forceinline__ void coarse_rows(const PoissonArgs& a, const FusedBlo
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
     if (lane == 0) __stcg(z + (t < PT / 32 ? zi : __ldg(a.cidx + k)), s);
   }
-}
-
-// V_new of node i from the solution, then the damped Picard update
-__device__ __forceinline__ double picard_update(const PoissonArgs& a, int i) {
-  const uint8_t c = __ldg(a.cls + i);
-  double vn;
-  if (c == NC_FREE) vn = (*(a.x + i));
-  else if (c == NC_DIR) vn = __ldg(a.Vfixed + i);
-  else {
-    int y = i / a.nx, x = i - y * a.nx;
-    int sy = y, sx = x;
-    if (x == a.nx - 1) {
-      sx = x - 1;  // right: copy (y, nx-2), which may itself be a top/bottom copy
-      uint8_t cs = __ldg(a.cls + sy * a.nx + sx);
-      if (cs == NC_NEU && !a.periodic) sy = (sy == 0) ? 1 : (sy == a.ny - 1 ? a.ny - 2 : sy);
-    } else if (y == 0) sy = 1;
-    else sy = a.ny - 2;
-    int j = sy * a.nx + sx;
-    uint8_t cj = __ldg(a.cls + j);
-    vn = (cj == NC_DIR) ? __ldg(a.Vfixed + j) : (*(a.x + j));
-  }
-  if (c != NC_FREE) __stcg(a.x + i, vn);
-  const double V = DADD(DMUL(a.omega_keep, (*(a.V + i))), DMUL(a.omega_new, vn));
-  __stcg(a.V + i, V);
-  return V;
 }
 
 template <bool RUNS>
