@@ -1734,10 +1734,13 @@ struct DeviceScope {
 // An upload runs as a pipeline: its copies on a stream of their own, the cell keys sorted while the
 // other arrays are on their way, each array re-ordered behind its own copy (a gather by itself
 // keeps more of its source in L2 than one of all arrays), the largest id found on the device.
-// Pinned arrays of n ions on 129 x 568 nodes, queued on one stream / so (single runs, 10% apart):
-// 100k 248 / 173 us, 250k 417 / 464, 500k 795 / 724, 1M 1143 / 892, 2M 1303 / 1362, 4M 2459 / 2043,
-// 16M 9908 / 7375; 48M ions and 16M electrons 59 ms as
-// copies, largest id on the host and sort one after another, 33 ms so (the copies alone 28.6).
+// Pinned arrays of n ions on 129 x 568 nodes, the calls one after another (medians of three runs of 50
+// uploads; copies, largest id on the host, sort / queued on one stream / so): 1k 160 / 152 / 120 us, 10k
+// 191 / 164 / 125, 100k 248 / 236 / 138, 250k 334 / 295 / 201, 500k 502 / 444 / 313, 1M 843 / 697 / 543, 2M
+// 1506 / 1213 / 1000, 4M 3093 / - / 1917.  Pageable: 100k 389 / 283 / 246, 1M 1753 / 1450 / 1421.  48M
+// ions and 16M electrons 59 ms before, 33 ms so (the copies alone 28.6).  A fresh simulator's first
+// upload of both species takes as long as before (80k ions and 20k electrons 2.1 / 2.1 ms,
+// medians of 40): its allocations are most of it.
 static int32_t upload_piped(Sim* s, int k, int n, const float* const* f, const uint8_t* cex, const uint32_t* id,
                             int bits, uint32_t* top) {
   if (!s->up) CK(cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking));
