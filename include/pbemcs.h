@@ -234,7 +234,8 @@ int32_t pb_sim_set_tile(pb_sim* s, int32_t particles_per_block);
 
 /* Upload the domain of build_domain (physics_engine.py:629-847): node masks, Dirichlet
  * values, electrode masks (bit g of gridmask = grid g), plus the state arrays to keep.
- * Host pointers.  Builds the node classes of build_sparse_matrix (:525-552) and the
+ * Host pointers.  A nonzero byte of isBound is an electrode cell (of these, only odd bytes conduct
+ * heat in the step; 1 is the ordinary value).  Builds the node classes of build_sparse_matrix (:525-552) and the
  * multigrid hierarchy.  keep_state != 0 keeps particles and damage. */
 int32_t pb_sim_set_domain(pb_sim* s, int32_t ny, int32_t nx, int32_t periodic, const uint8_t* isBound,
                           const double* V_fixed, const uint16_t* gridmask, int32_t ngrids, const double* V,

@@ -1739,7 +1739,7 @@ struct DeviceScope {
 // 191 / 164 / 125, 100k 248 / 236 / 138, 250k 334 / 295 / 201, 500k 502 / 444 / 313, 1M 843 / 697 / 543, 2M
 // 1506 / 1213 / 1000, 4M 3093 / - / 1917.  Pageable: 100k 389 / 283 / 246, 1M 1753 / 1450 / 1421.  48M
 // ions and 16M electrons 59 ms before, 33 ms so (the copies alone 28.6).  A fresh simulator's first
-// upload of both species takes as long as before (80k ions and 20k electrons 2.1 / 2.1 ms,
+// upload of both species takes as long as before (80k ions and 20k electrons 2.1 / 2.2 ms,
 // medians of 40): its allocations are most of it.
 static int32_t upload_piped(Sim* s, int k, int n, const float* const* f, const uint8_t* cex, const uint32_t* id,
                             int bits, uint32_t* top) {
