@@ -955,7 +955,8 @@ __device__ __forceinline__ int level_share(const PoissonArgs& a, int l) {
   return 32 * (((a.lev[l].ny * a.lev[l].nx + 31) / 32 + a.nblk - 1) / a.nblk);
 }
 
-template <bool RUNS>
+// FILL: the tables' contents too; else the layout only.
+template <bool RUNS, bool FILL>
 __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c1, FusedBlock& B, FusedLevel* lv) {
   const int tid = (int)threadIdx.x, N = a.ny * a.nx, nx = a.nx, last = a.nlevels - 1;
   const MgLevel &L1 = a.lev[1], &L2 = a.lev[2];
@@ -994,17 +995,17 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
   for (int l = 2; l <= last; ++l) {
     const int sh = level_share(a, l), Nl = a.lev[l].ny * a.lev[l].nx, lx = a.lev[l].nx;
     int* const t = takei(sh);
-    for (int q = tid; q < sh; q += PT) {
+    for (int q = tid; FILL && q < sh; q += PT) {
       const int i = ((q >> 5) * a.nblk + gbid(a)) * 32 + (q & 31), y = i / lx;
       t[q] = i < Nl ? (y << 16) | (i - y * lx) : -1;
     }
-    if (tid == 0) {
+    if (FILL && tid == 0) {
       lv[l].L = a.lev[l];
       lv[l].yx = t;
       lv[l].share = sh;
     }
   }
-  if (tid == 0) lv[1].L = a.lev[1];
+  if (FILL && tid == 0) lv[1].L = a.lev[1];
   // Level 1 under the runs: a run is one or two row segments (it may cross a row's end, and is no
   // longer than a row); the patch of a segment is the coarse nodes that its two rows and columns
   // on every side interpolate from.  seg: first run column, fine row, coarse origin, size, place
@@ -1020,7 +1021,7 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     nz = (Yb - Ya + 1) * sw;
     seg_c0[0] = Ya << 16 | Xa;
     seg_w[0] = sw;
-    for (int k = tid; k < nz; k += PT) {
+    for (int k = tid; FILL && k < nz; k += PT) {
       const int y = Ya + k / sw, x = Xa + k % sw;
       B.zn[k] = ((y - 2 * I0 + 2) * B.W1 + x - 2 * J0 + 2) << 16 | (((y >> 1) - I0 + 2) * B.W2 + (x >> 1) - J0 + 2);
     }
@@ -1040,7 +1041,7 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     const int sw = Xb - Xa + 1, cnt = (Yb - Ya + 1) * sw;
     seg_c0[q] = Ya << 16 | Xa;
     seg_w[q] = sw;
-    for (int k = tid; k < cnt; k += PT) B.zn[nz + k] = (Ya + k / sw) << 16 | (Xa + k % sw);
+    for (int k = tid; FILL && k < cnt; k += PT) B.zn[nz + k] = (Ya + k / sw) << 16 | (Xa + k % sw);
     nz += cnt;
   }
   B.nz = nz;
@@ -1054,12 +1055,15 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     B.zj = takei(B.n2);
     B.z2 = take(B.n2);
     B.uf = takei(B.np);
-    for (int k = tid; k < B.n2; k += PT) {
+    for (int k = tid; FILL && k < B.n2; k += PT) {
       const int y = I0 - 2 + k / B.W2, x = J0 - 2 + k % B.W2;
       B.zj[k] = (unsigned)y < (unsigned)L2.ny && (unsigned)x < (unsigned)L2.nx ? y * L2.nx + x : -1;
     }
   }
   B.crow = f;
+  const int nc = __ldg(a.nc_dev), lane = tid & 31;
+  B.crows = min((int)((size_t)a.croom / max(nc, 1)), (nc + a.nblk - 1) / a.nblk);
+  if (!FILL) return;
   __syncthreads();
   for (int k = tid; k < nz; k += PT) {
     const int i = RUNS ? (B.zn[k] >> 16) * L1.nx + (B.zn[k] & 0xFFFF)
@@ -1122,8 +1126,6 @@ __device__ __forceinline__ void fused_tables(const PoissonArgs& a, int c0, int c
     B.uf[k] = uf;
     B.ud[k] = d;
   }
-  const int nc = __ldg(a.nc_dev), lane = tid & 31;
-  B.crows = min((int)((size_t)a.croom / max(nc, 1)), (nc + a.nblk - 1) / a.nblk);
   for (int t = tid >> 5; t < B.crows; t += PT / 32) {
     const int k = t * a.nblk + gbid(a);
     if (k >= nc) break;
@@ -1379,8 +1381,8 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
 
   __shared__ FusedLevel lv[MG_MAX_LEVELS];
   FusedBlock B;
-  fused_tables<RUNS>(a, c0, c1, B, lv);
-  __syncthreads();
+  fused_tables<RUNS, false>(a, c0, c1, B, lv);
+  bool laid = false;  // the tables, 10 to 15 us, are filled by the first linear solve that needs an iteration
   const int nc = __ldg(a.nc_dev);
   int ci[2], zi = -1;
 #pragma unroll
@@ -1458,6 +1460,12 @@ __device__ __forceinline__ void poisson_body_fused(const PoissonArgs& a) {
     tmark(a, 17);
     const double target2 = a.tol * a.tol * fnorm2;
 
+    if (!laid && rnorm2 > target2 && fnorm2 > 0.0) {
+      laid = true;
+      FusedBlock t;
+      fused_tables<RUNS, true>(a, c0, c1, t, lv);
+      __syncthreads();
+    }
     for (int outer = 0; outer < a.max_outer && rnorm2 > target2 && fnorm2 > 0.0; ++outer) {
       n_outer += 1;
       double rz_old = 0.0, rr0 = rnorm2;
