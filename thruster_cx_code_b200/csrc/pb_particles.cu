@@ -695,7 +695,9 @@ __global__ void __cluster_dims__(DEP_C, 1, 1) __launch_bounds__(1024)
       if (r < n4) { add(Z.x, W.x); add(Z.y, W.y); add(Z.z, W.z); add(Z.w, W.w); }
     }
   }
-  for (unsigned i = (unsigned)done + t0; i < (unsigned)n; i += stride) add(x[i], y[i]);
+  x += done;
+  y += done;
+  for (unsigned i = t0; i < (unsigned)(n - done); i += stride) add(x[i], y[i]);
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   const uint32_t base = smem_addr(hist);
   uint32_t at[DEP_C];
