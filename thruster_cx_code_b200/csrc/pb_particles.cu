@@ -601,21 +601,43 @@ __device__ __forceinline__ int deposit_cell(float x, float y, float dxf, float d
 // neighbouring lanes mostly share cells (particles sorted by cell) aggregates equal cells
 // before the atomics; otherwise one atomic per particle: __match_any_sync over distinct cells
 // takes one round per cell and bound the kernel (6M scattered ions on 257 x 1025: 53 us,
-// match unit 79% busy, DRAM 11%; 42 us so, 160 G atomics/s).
-__device__ __forceinline__ void count_add(int* cnt, int cell, bool valid) {
-  const int left = __shfl_up_sync(0xFFFFFFFFu, cell, 1);
-  const unsigned same = __ballot_sync(0xFFFFFFFFu, valid && left == cell);
-  if (__popc(same) >= 16) warp_count_add(cnt, cell, valid);
-  else if (valid) atomicAdd(cnt + cell, 1);
-}
+// match unit 79% busy, DRAM 11%; 42 us so, 160 G atomics/s).  Aggregation also pays where the
+// warp's particles lie in few cells without being sorted, as atomics on few words take turns:
+// warps whose tests often found a particle of another lane's in a cell of theirs (some 200 cells
+// or fewer) aggregate too: 20M ions scattered over 20, 60 and 150 cells take 2117, 1204 and 942 us
+// with plain atomics, 954, 917 and 890 us so; over all of 257 x 1025 144 and 142 us.
+struct CountCrowd {
+  int met = 0, turn = 0;
+  bool on = false;
+  // the warp's particles in cells c[0..N); tested every fourth turn
+  template <int N>
+  __device__ __forceinline__ void add(int* cnt, const int (&c)[N], bool valid) {
+    if ((turn++ & 3) == 0) {
+      const int left = __shfl_up_sync(0xFFFFFFFFu, c[0], 1), far = __shfl_xor_sync(0xFFFFFFFFu, c[0], 16);
+      bool meets = false;
+#pragma unroll
+      for (int k = 0; k < N && k < 2; ++k) meets |= far == c[k];
+      met += __any_sync(0xFFFFFFFFu, valid && meets) ? 16 : 0;
+      on = __popc(__ballot_sync(0xFFFFFFFFu, valid && left == c[0])) >= 16 || met >= turn;  // a quarter of the tests
+    }
+    if (on) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) warp_count_add(cnt, c[k], valid);
+    } else if (valid) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) atomicAdd(cnt + c[k], 1);
+    }
+  }
+};
 
-__global__ void __launch_bounds__(256) k_count_cells(const float* __restrict__ x, const float* __restrict__ y,
+__global__ void __launch_bounds__(256, 8) k_count_cells(const float* __restrict__ x, const float* __restrict__ y,
                                                      const int* n_dev, int n_host, int start, int* cnt, int nx, int ny,
                                                      float dxf, float dyf) {
   pdl_enter();
   const int n = n_dev ? *n_dev : n_host;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   int done = start;
+  CountCrowd crowd;
   if (start == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0) {
     const int n4 = n >> 2, lane = threadIdx.x & 31;
     done = n4 << 2;
@@ -627,18 +649,16 @@ __global__ void __launch_bounds__(256) k_count_cells(const float* __restrict__ x
         X = __ldg(reinterpret_cast<const float4*>(x) + q);
         Y = __ldg(reinterpret_cast<const float4*>(y) + q);
       }
-      const int c0 = deposit_cell(X.x, Y.x, dxf, dyf, nx, ny), c1 = deposit_cell(X.y, Y.y, dxf, dyf, nx, ny);
-      const int c2 = deposit_cell(X.z, Y.z, dxf, dyf, nx, ny), c3 = deposit_cell(X.w, Y.w, dxf, dyf, nx, ny);
-      count_add(cnt, c0, v);
-      count_add(cnt, c1, v);
-      count_add(cnt, c2, v);
-      count_add(cnt, c3, v);
+      const int c[4] = {deposit_cell(X.x, Y.x, dxf, dyf, nx, ny), deposit_cell(X.y, Y.y, dxf, dyf, nx, ny),
+                        deposit_cell(X.z, Y.z, dxf, dyf, nx, ny), deposit_cell(X.w, Y.w, dxf, dyf, nx, ny)};
+      crowd.add(cnt, c, v);
     }
   }
   for (unsigned i0 = (unsigned)done + t0 - (threadIdx.x & 31); i0 < (unsigned)n; i0 += stride) {
     const unsigned i = i0 + (threadIdx.x & 31);
     const bool v = i < (unsigned)n;
-    count_add(cnt, v ? deposit_cell(x[i], y[i], dxf, dyf, nx, ny) : 0, v);
+    const int c[1] = {v ? deposit_cell(x[i], y[i], dxf, dyf, nx, ny) : -1};
+    crowd.add(cnt, c, v);
   }
 }
 
