@@ -2353,11 +2353,20 @@ int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float*
 // global atomics: up to DEPOSIT_ONE_MAX particles in one launch (two calls of 190k and 60k
 // particles take 35 us so and 36 us with the count kernels; at 100k and below the launches and
 // the scratch saved decide), and from DEPOSIT_MANY_MIN on, where the atomics on a small grid's
-// cells collide (two calls of 1.1M each on 65 x 284: 47 us; of 900k each by atomics 51 us).
+// cells collide, with more particles on larger grids, whose atomics collide less and whose histograms
+// take longer to clear and add up: from the square of the cells / 600 on.  Scattered particles,
+// clusters against counts (us): 65 x 284 nodes 1M 23 / 24 to 29 (two boxes), 4M 31 / 63 to 82; 99 x 260 1M
+// 25 / 21, 2M 30 / 35; 129 x 300 1M 31 / 18, 2M 38 / 28 to 34, 4M 46 / 49 to 61; 160 x 320 1M 31 / 16, 4M 46 / 43 to
+// 53, 8M 62 / 71 to 86.  Particles sorted by cell are counted faster than that at every size (4M on
+// 65 x 284 31 / 20, on 160 x 320 46 / 23), but the host cannot tell; a mark from the device cost
+// scattered ones 2 to 5%.
 constexpr int DEPOSIT_ONE_MAX = 100000;
-constexpr int DEPOSIT_MANY_MIN = 1000000;
+constexpr int DEPOSIT_MANY_MIN = 1000000, DEPOSIT_MANY_CELLS2 = 600;
 constexpr int DEPOSIT_CLUSTERS = 18;   // of eight blocks: 144 SMs
 constexpr size_t DEPOSIT_CLUSTER_SMEM = 200 * 1024;
+static bool deposit_many(int n, int G) {
+  return n >= DEPOSIT_MANY_MIN && (long long)n * DEPOSIT_MANY_CELLS2 >= (long long)G * G;
+}
 static size_t deposit_smem(int G) { return ((size_t)G + 3) / 4 * 16; }
 
 // counts cleared, filled and rounded into rho
@@ -2417,7 +2426,7 @@ int32_t pb_accumulate_rho(const float* x, const float* y, float* rho, int32_t nu
   }
   int* cnt = nullptr;
   CK(scratch_alloc((void**)&cnt, (size_t)G * sizeof(int), st));
-  const int32_t rc = deposit_counts(x, y, rho, num_p, dx, dy, nx, ny, charge_density, cnt, st, clusters && num_p >= DEPOSIT_MANY_MIN);
+  const int32_t rc = deposit_counts(x, y, rho, num_p, dx, dy, nx, ny, charge_density, cnt, st, clusters && deposit_many(num_p, G));
   const cudaError_t ef = cudaFreeAsync(cnt, st);
   if (rc) return rc;
   CK(ef);
