@@ -103,16 +103,26 @@ class ClockSampler:
         self.gpu = gpu
         self.proc = None
         self.lines = []
+        self.first = 0
 
     def start(self):
+        """Returns once samples arrive (the timed region, 0.15 s, is shorter than nvidia-smi's start-up)."""
         try:
             self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.gpu), f"--query-gpu={self.FIELDS}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"],
+                                          "--format=csv,noheader,nounits", "-lms", "50"],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
         except Exception:
             self.proc = None
+            return
+        end = time.monotonic() + 10.0
+        while not self.lines and self.proc.poll() is None and time.monotonic() < end:
+            time.sleep(0.005)
+
+    def region(self):
+        """The timed region begins: earlier samples do not count."""
+        self.first = len(self.lines)
 
     def _read(self):
         for line in self.proc.stdout:
@@ -128,7 +138,7 @@ class ClockSampler:
             self.proc.kill()
         sm, mx, reasons = [], None, set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for ln in self.lines:
+        for ln in self.lines[self.first:]:
             p = [x.strip() for x in ln.split(",")]
             if len(p) < 9:
                 continue
@@ -306,14 +316,15 @@ def gpu_arm(args):
         dist.init_process_group("nccl", timeout=datetime.timedelta(seconds=300))
     _lib.load()
     sim, params = make_gpu_sim(args.workload, local, seed=1000 + rank)
+    clocks = ClockSampler(local)
+    clocks.start()  # ahead of the warm-up, which leaves the GPU at its clocks
     for _ in range(args.warmup):
         sim.step(params)
     K = args.steps
-    clocks = ClockSampler(local)
     if world > 1:
         torch.distributed.barrier()
     torch.cuda.synchronize()
-    clocks.start()
+    clocks.region()
     run = timed_run(sim, params, K)
     torch.cuda.synchronize()
     clk = clocks.stop()
