@@ -2310,8 +2310,10 @@ int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float*
   // grid and three more launches.  Measured, direct against packed (us): 65 x 284 nodes 20
   // against 26 at 400k particles, 41 against 26 at 1M; 257 x 1025 27 against 19 (27 with a B
   // field) at 400k, 59 against 23 (39) at 1M; 513 x 2049 60 against 33 (72) at 1M, 225 against
-  // 61 (132) at 4M.  So from 600k particles and 1.5 a cell.  A capturing stream keeps the one
-  // launch, which needs no memory.
+  // 61 (132) at 4M.  So from 600k particles and 1.5 a cell.  Only grids of under a thousand cells,
+  // whose fields stay in L1, lose with a B field: 9 x 17 12 against 20 at 600k, 17 against 24 at 1M,
+  // 31 against 33 at 2M; without one they gain from 1M on (23 against 15).  A capturing stream keeps
+  // the one launch, which needs no memory.
   if (num_p >= PUSH_PACK_MIN && (long long)num_p * 2 >= 3 * cells && cells <= PUSH_PACK_CELLS && !stream_capturing(st)) {
     const size_t fl = ((PUSH_FLAGS * sizeof(unsigned) + 255) / 256) * 256;
     char* ws = nullptr;
