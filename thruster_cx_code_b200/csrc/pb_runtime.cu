@@ -2357,7 +2357,7 @@ int32_t pb_push_particles_boris(float* x, float* y, float* vx, float* vy, float*
 // the scratch saved decide), and from DEPOSIT_MANY_MIN on, where the atomics on a small grid's
 // cells collide, with more particles on larger grids, whose atomics collide less and whose histograms
 // take longer to clear and add up: from the square of the cells / 600 on.  Scattered particles,
-// clusters against counts (us): 65 x 284 nodes 1M 23 / 24 to 29 (two boxes), 4M 31 / 63 to 82; 99 x 260 1M
+// clusters against counts (us): 65 x 284 nodes 1M 23 / 24 to 29 (two GPUs), 4M 31 / 63 to 82; 99 x 260 1M
 // 25 / 21, 2M 30 / 35; 129 x 300 1M 31 / 18, 2M 38 / 28 to 34, 4M 46 / 49 to 61; 160 x 320 1M 31 / 16, 4M 46 / 43 to
 // 53, 8M 62 / 71 to 86.  Particles sorted by cell are counted faster than that at every size (4M on
 // 65 x 284 31 / 20, on 160 x 320 46 / 23), but the host cannot tell; a mark from the device cost
