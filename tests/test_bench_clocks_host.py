@@ -28,10 +28,13 @@ def test_short_region_is_sampled(tmp_path, monkeypatch):
     s = bench.ClockSampler(0)
     s.start()
     s.region()
-    time.sleep(0.15)
+    t0 = time.monotonic()
+    while not s.lines[s.first:] and time.monotonic() < t0 + 5.0:  # a loaded host may be late
+        time.sleep(0.15)
     got = s.stop()
     assert (got["sm_mhz"], got["sm_max_mhz"], got["reasons"]) == (1900.0, 1965.0, ["sw_power_cap"]), got
-    assert 1 <= got["samples"] <= 6, got  # none of the time before the region
+    # none of the time before the region
+    assert 1 <= got["samples"] <= (time.monotonic() - t0) / 0.05 + 2, got
 
 
 def test_without_nvidia_smi(tmp_path, monkeypatch):
